@@ -22,13 +22,16 @@
 
 #include "pt_device.cuh"
 #include "pt_kernels.h"
+#include "slab.h"
 
 namespace ptg {
 
 // Minimum resident blocks per SM requested from the register allocator for the
-// trace (extend/shadow) and shade stages; 1 leaves the choice to the compiler.
+// trace (extend/shadow) and shade stages; 1 leaves the choice to the compiler. Trace: 7
+// blocks of 72 registers; 8 of 64 (which spill), 6 and 5 measured 17.65, 17.30 and 17.85 ms
+// against 16.90 for the closest hits of the 1.0M-triangle 1080p frame.
 #ifndef PT_TRACE_MIN_BLOCKS
-#define PT_TRACE_MIN_BLOCKS 8
+#define PT_TRACE_MIN_BLOCKS 7
 #endif
 #ifndef PT_SHADE_MIN_BLOCKS
 #define PT_SHADE_MIN_BLOCKS 1
@@ -48,34 +51,6 @@ __device__ __forceinline__ void PixelOfIndex(int q, int W, int H, int rows, int&
     y = y0 + r % hb;
 }
 
-// Three-input maximum and minimum (max.f32 / min.f32 with three sources, sm_100 and
-// later); a NaN operand is ignored, as by fmaxf / fminf.
-__device__ __forceinline__ float Max3(float a, float b, float c) {
-    float d;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
-__device__ __forceinline__ float Min3(float a, float b, float c) {
-    float d;
-    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
-
-// Box test against [tmin, tmax]; returns the entry distance. Each plane distance is
-// one fused multiply-add, plane * inv - oi with oi = o * inv. Its rounding
-// (a few units in the last place of the origin's and the distance's coordinates) is
-// far inside the 2^-18 widening of the child boxes, so no hit box is missed.
-__device__ __forceinline__ bool SlabFast(float4 a, float4 b, V3 oi, V3 inv, float tmin, float tmax,
-                                         float& tEnter) {
-    const float tx0 = fmaf(a.x, inv.x, -oi.x), tx1 = fmaf(a.w, inv.x, -oi.x);
-    const float ty0 = fmaf(a.y, inv.y, -oi.y), ty1 = fmaf(b.x, inv.y, -oi.y);
-    const float tz0 = fmaf(a.z, inv.z, -oi.z), tz1 = fmaf(b.y, inv.z, -oi.z);
-    const float tn = Max3(fminf(tx0, tx1), fminf(ty0, ty1), fmaxf(fminf(tz0, tz1), tmin));
-    const float tf = Min3(fmaxf(tx0, tx1), fmaxf(ty0, ty1), fminf(fmaxf(tz0, tz1), tmax));
-    tEnter = tn;
-    return tn <= tf;
-}
-
 __device__ __forceinline__ int WarpAppend(int* counter, bool pred) {
     const unsigned active = __activemask();
     const unsigned mask = __ballot_sync(active, pred);
@@ -91,12 +66,10 @@ __device__ __forceinline__ int WarpAppend(int* counter, bool pred) {
 // Warp-persistent traversal with dynamic ray fetch: each warp pulls rays from a
 // queue counter and refills its idle lanes whenever a quarter of the warp has
 // finished, so long rays do not hold a warp of finished lanes (the load
-// imbalance of incoherent secondary rays). One node visit per loop iteration.
+// imbalance of incoherent secondary rays). Bound by issue and by the warps' own
+// latency: of 4M incoherent rays, 8 of 32 lanes were active per instruction, 70% of
+// issue slots busy and the L1 data pipe at 80%.
 constexpr unsigned kFullMask = 0xffffffffu;
-#ifndef PT_REFILL_LANES
-#define PT_REFILL_LANES 8
-#endif
-constexpr int kRefillLanes = PT_REFILL_LANES;
 
 struct LaneRay {
     V3 o, d, inv;
@@ -105,10 +78,21 @@ struct LaneRay {
     bool anyHit;
     const float4* nodes;  // the lane's 4-wide tree (rays of different jobs share a warp)
     const float4* tris;
+    int nearX, nearY, nearZ;  // byte offsets in a node of the planes the ray meets first
 #if PT_CHECK
     int numWide, numTris;  // bounds of nodes and tris, tested before every access
 #endif
+    __device__ __forceinline__ void Start();
 };
+__device__ __forceinline__ void LaneRay::Start() {
+    inv = ExactRecip(d);
+    tBest = tmax;
+    best = -1;
+    constexpr int kP = 4 * kWide;  // bytes of one plane of a node's children
+    nearX = 3 * kP * UpperFirst(inv.x, o.x * inv.x);
+    nearY = 3 * kP * UpperFirst(inv.y, o.y * inv.y) + kP;
+    nearZ = 3 * kP * UpperFirst(inv.z, o.z * inv.z) + 2 * kP;
+}
 
 __device__ __forceinline__ void SortPair(float& ta, int& ca, float& tb, int& cb) {
     if (tb < ta) {
@@ -123,18 +107,21 @@ __device__ __forceinline__ void SortPair(float& ta, int& ca, float& tb, int& cb)
 
 // Entries of the traversal stack kept in shared memory per thread; deeper ones go
 // to local memory. Shared entries are entry-major with one column per thread of
-// the 128-thread block, so a warp's accesses always fall in 32 distinct banks.
+// the 128-thread block, so a warp's accesses always fall in 32 distinct banks. 8 entries
+// leave more of the SM's memory to L1 and to the other stream's blocks than 12 or 16: a
+// 2.2M-triangle 4K terrain frame took 27.66, 27.89 and 27.91 ms.
 #ifndef PT_SMEM_STACK
-#define PT_SMEM_STACK 16
-#endif
-// 1: a warp steps every lane through inner nodes until it reaches a leaf, then
-// intersects the lanes' leaves together; 0: one node or leaf per lane per step.
-// Both visit the same nodes and leaves in the same order for every ray.
-#ifndef PT_WHILE_WHILE
-#define PT_WHILE_WHILE 1
+#define PT_SMEM_STACK 8
 #endif
 constexpr int kTraceBlock = 128;
+constexpr int kTraceWarps = kTraceBlock / 32;
 constexpr int kSmemStack = PT_SMEM_STACK;
+// A warp leaves the inner-node steps for its leaves once at most this many of its lanes
+// still hold an inner node (they wait): 2, 4, 8 and 12 measured 17.97, 17.77, 17.77 and
+// 17.79 ms for the closest hits of the 1.0M-triangle 1080p frame, against 18.90 with every
+// lane stepped to a leaf (0), and 748, 745 and 750 us for 4M incoherent rays (4, 8, 12)
+// against 787.
+constexpr int kLeafLanes = 4;
 constexpr int kDone = INT_MIN;  // no further item (never a child code of a visited slot)
 
 struct TravStack {
@@ -218,38 +205,32 @@ __device__ __forceinline__ void VisitInner(LaneRay& r, TravStack& stk, int& cur,
         return;
     }
 #endif
-    const float4* n = r.nodes + (kWideFloats / 4) * (size_t)cur;
-    float b[6][K];
-#pragma unroll
-    for (int a = 0; a < 6; a++)
-#pragma unroll
-        for (int j = 0; j < Q; j++) {
-            const float4 v = __ldg(n + a * Q + j);
-            b[a][4 * j] = v.x;
-            b[a][4 * j + 1] = v.y;
-            b[a][4 * j + 2] = v.z;
-            b[a][4 * j + 3] = v.w;
-        }
-    int c[K];
-#pragma unroll
-    for (int j = 0; j < Q; j++) {
-        const int4 v = __ldg(reinterpret_cast<const int4*>(n + 6 * Q + j));
-        c[4 * j] = v.x;
-        c[4 * j + 1] = v.y;
-        c[4 * j + 2] = v.z;
-        c[4 * j + 3] = v.w;
-    }
+    const char* n = reinterpret_cast<const char*>(r.nodes) + 4 * kWideFloats * (size_t)cur;
+    constexpr int kP = 4 * K;  // bytes of one plane of the K children
+    const char* plane[6] = {n + r.nearX,          n + r.nearY,          n + r.nearZ,
+                            n + 3 * kP - r.nearX, n + 5 * kP - r.nearY, n + 7 * kP - r.nearZ};
     const float inf = __int_as_float(0x7f800000);
     const V3 oi = r.o * r.inv;
     float t[K];
+    int c[K];
 #pragma unroll
-    for (int i = 0; i < K; i++) {
-        float te;
+    for (int j = 0; j < Q; j++) {
+        float4 v[6];
+#pragma unroll
+        for (int a = 0; a < 6; a++) v[a] = __ldg(reinterpret_cast<const float4*>(plane[a]) + j);
+        const int4 code = __ldg(reinterpret_cast<const int4*>(n + 6 * kP) + j);
+        c[4 * j] = code.x;
+        c[4 * j + 1] = code.y;
+        c[4 * j + 2] = code.z;
+        c[4 * j + 3] = code.w;
         // an empty slot's box lies at +infinity on every plane and is never hit
-        t[i] = SlabFast(make_float4(b[0][i], b[1][i], b[2][i], b[3][i]),
-                        make_float4(b[4][i], b[5][i], 0.f, 0.f), oi, r.inv, 0.0f, r.tBest, te)
-                 ? te
-                 : inf;
+        auto slab = [&](float nx, float ny, float nz, float fx, float fy, float fz) {
+            return SlabEntry(nx, ny, nz, fx, fy, fz, r.inv.x, r.inv.y, r.inv.z, oi.x, oi.y, oi.z, r.tBest);
+        };
+        t[4 * j] = slab(v[0].x, v[1].x, v[2].x, v[3].x, v[4].x, v[5].x);
+        t[4 * j + 1] = slab(v[0].y, v[1].y, v[2].y, v[3].y, v[4].y, v[5].y);
+        t[4 * j + 2] = slab(v[0].z, v[1].z, v[2].z, v[3].z, v[4].z, v[5].z);
+        t[4 * j + 3] = slab(v[0].w, v[1].w, v[2].w, v[3].w, v[4].w, v[5].w);
     }
     if (kAnyHit && K == 4) {
         // the nearest into slot 0
@@ -258,6 +239,19 @@ __device__ __forceinline__ void VisitInner(LaneRay& r, TravStack& stk, int& cur,
         SortPair(t[0], c[0], t[2], c[2]);
         if (t[0] == inf) {
             cur = stk.PopCode();
+            return;
+        }
+        if (stk.sp <= kSmemStack - (K - 1)) {  // room in shared memory: no branch per push
+            int* e = stk.code + stk.sp * kTraceBlock + threadIdx.x;
+#pragma unroll
+            for (int i = K - 1; i >= 1; i--) {
+                *e = c[i];
+                if (t[i] != inf) {
+                    e += kTraceBlock;
+                    stk.sp++;
+                }
+            }
+            cur = c[0];
             return;
         }
         if (stk.sp > kWaveStackDepth - (K - 1)) {  // room for K - 1 pushes
@@ -287,6 +281,19 @@ __device__ __forceinline__ void VisitInner(LaneRay& r, TravStack& stk, int& cur,
     }
     if (t[0] == inf) {
         cur = stk.Pop(r.tBest);
+        return;
+    }
+    if (stk.sp <= kSmemStack - (K - 1)) {  // room in shared memory: no branch per push
+        int2* e = stk.ent + stk.sp * kTraceBlock + threadIdx.x;
+#pragma unroll
+        for (int i = K - 1; i >= 1; i--) {
+            *e = make_int2(c[i], __float_as_int(t[i]));
+            if (t[i] != inf) {
+                e += kTraceBlock;
+                stk.sp++;
+            }
+        }
+        cur = c[0];
         return;
     }
     if (stk.sp > kWaveStackDepth - (K - 1)) {  // room for K - 1 pushes
@@ -332,6 +339,11 @@ __device__ void TraceQueue(Q& q, int n, int* fetch, int& err) {
     __shared__ int sCode[kAnyHit && kSmemStack > 0 ? kSmemStack * kTraceBlock : 1];
     const int lane = threadIdx.x & 31;
     const unsigned lowerLanes = (1u << lane) - 1u;
+    const int warps = gridDim.x * kTraceWarps;
+    // A queue shorter than the grid's lanes is spread over all its warps: fewer rays a warp
+    // diverge less, and the launch lasts as long as its slowest warp. A 128x72 1-spp frame of
+    // nine such queues took 356 us against 478 with full warps.
+    const int lim = min(32, max(1, (n + warps - 1) / warps));
     LaneRay r;
     int idx = -1;
     bool active = false;
@@ -340,50 +352,43 @@ __device__ void TraceQueue(Q& q, int n, int* fetch, int& err) {
     stk.code = sCode;
     stk.sp = 0;
     int cur = kDone;
-    bool exhausted = false;  // warp-uniform
+    bool exhausted = n <= 0;  // warp-uniform
     for (;;) {
         const unsigned idle = __ballot_sync(kFullMask, !active);
         const int nIdle = __popc(idle);
-        if (!exhausted && (nIdle >= kRefillLanes || idle == kFullMask)) {
-            int base = 0;
-            if (lane == 0) base = atomicAdd(fetch, nIdle);
-            base = __shfl_sync(kFullMask, base, 0);
-            exhausted = base + nIdle >= n;
-            if (!active) {
-                const int i = base + __popc(idle & lowerLanes);
-                if (i < n) {
-                    idx = i;
-                    q.Load(i, r);
-                    r.inv = ExactRecip(r.d);
-                    r.tBest = r.tmax;
-                    r.best = -1;
-                    stk.sp = 0;
-                    if (r.nodes) {
-                        cur = 0;  // wide root
-                        active = true;
-                    } else {
-                        q.Finish(i, r);
-                    }
+        if (!exhausted && 32 - nIdle <= (3 * lim) / 4) {
+            const int take = min(nIdle, lim - (32 - nIdle));
+            int first = 0;
+            if (lane == 0) first = atomicAdd(fetch, take);
+            first = __shfl_sync(kFullMask, first, 0);
+            exhausted = first + take >= n;
+            const int k = __popc(idle & lowerLanes);
+            if (!active && k < take && first + k < n) {
+                idx = first + k;
+                q.Load(idx, r);
+                r.Start();
+                stk.sp = 0;
+                if (r.nodes) {
+                    cur = 0;  // wide root
+                    active = true;
+                } else {
+                    q.Finish(idx, r);
                 }
             }
         }
-        if (!__any_sync(kFullMask, active)) {
+        const unsigned busy = __ballot_sync(kFullMask, active);
+        if (busy == 0) {
             if (exhausted) break;
             continue;
         }
-#if PT_WHILE_WHILE
-        const unsigned busy = __ballot_sync(kFullMask, active);
-#endif
         if (active) {
             bool done = false;
-#if PT_WHILE_WHILE
-            while (cur >= 0) VisitInner<kAnyHit>(r, stk, cur, err);
-            __syncwarp(busy);  // the lanes' leaves are intersected together
-            if (cur != kDone) done = VisitLeaf<kAnyHit>(r, stk, cur, err);
-#else
-            if (cur >= 0) VisitInner<kAnyHit>(r, stk, cur, err);
-            else if (cur != kDone) done = VisitLeaf<kAnyHit>(r, stk, cur, err);
-#endif
+            for (;;) {
+                if (cur >= 0) VisitInner<kAnyHit>(r, stk, cur, err);
+                const unsigned in = __ballot_sync(busy, cur >= 0);
+                if (in == 0 || (__popc(in) <= kLeafLanes && in != busy)) break;
+            }
+            if (cur < 0 && cur != kDone) done = VisitLeaf<kAnyHit>(r, stk, cur, err);
             if (done || cur == kDone) {
                 q.Finish(idx, r);
                 active = false;
@@ -873,9 +878,7 @@ struct ShadowQueue {
 // One ray traversed by one thread (the tail kernel's form): the same node and leaf
 // order as TraceQueue gives the ray.
 __device__ __forceinline__ void TraceOne(LaneRay& r, TravStack& stk, int& err) {
-    r.inv = ExactRecip(r.d);
-    r.tBest = r.tmax;
-    r.best = -1;
+    r.Start();
     stk.sp = 0;
     if (!r.nodes) return;
     int cur = 0;  // wide root
