@@ -342,6 +342,7 @@ struct ONB {  // Math/OrthonormalBasis.cpp:10-62
 };
 
 // ---------------------------------------------------------------- camera
+__device__ __forceinline__ bool IsNegZero(float x) { return __float_as_uint(x) == 0x80000000u; }
 // Camera::GenerateRay (Core/Camera.cpp:52-91); (r0,r1) sensor, (r2,r3) lens
 template <class M>
 __device__ __forceinline__ Ray GenerateRay(const DevCamera& c, int i, int j, int W, int H, float r0,
@@ -352,10 +353,15 @@ __device__ __forceinline__ Ray GenerateRay(const DevCamera& c, int i, int j, int
     const float v = (j + r1) / H - 0.5f;
     const V3 onSensor = pos + right * u * c.hPerf * c.focusDist * aspect +
                         -up * v * c.hPerf * c.focusDist + fwd * c.focusDist;
-    const float r = sqrtf(r2);
-    const float theta = 2.0f * kPi * r3;
-    const V3 onLens = pos + right * 0.5f * c.aperture * r * M::Cos(theta) +
-                      -up * 0.5f * c.aperture * r * M::Sin(theta);
+    // a pinhole's lens offsets are zeros, which change no component but a negative zero: their
+    // sine and cosine are not needed (in FP64 about 2800 cycles per sample)
+    V3 onLens = pos;
+    if (c.aperture != 0.0f || IsNegZero(pos.x) || IsNegZero(pos.y) || IsNegZero(pos.z)) {
+        const float r = sqrtf(r2);
+        const float theta = 2.0f * kPi * r3;
+        onLens = pos + right * 0.5f * c.aperture * r * M::Cos(theta) +
+                 -up * 0.5f * c.aperture * r * M::Sin(theta);
+    }
     Ray ray;
     ray.o = onLens;
     ray.d = M::Norm(onSensor - onLens);

@@ -23,14 +23,14 @@ int NumTiles(const DevSettings& st);
 cudaError_t ProbeL2Read(const void* buf, size_t bytes, int passes, int reps, float* sink,
                         cudaStream_t stream, float* ms);
 
-// Replay: one thread per tile in [tileBegin, tileEnd). stackScratch holds
+// Replay: one warp per tile in [tileBegin, tileEnd). stackScratch holds
 // (tileEnd - tileBegin) * S.stackDepth ints. status receives error bits (OR).
 cudaError_t LaunchReplay(const DevScene& S, const DevCamera& C, const DevSettings& st, float* film,
                          int* stackScratch, int* status, int tileBegin, int tileEnd,
                          cudaStream_t stream);
 
 // AOV pass (0 UV, 1 denoising albedo, 2 denoising normal) of tiles [tileBegin, tileEnd):
-// one thread per tile with the reference's per-tile stream; dspp = numSppForDenoising.
+// one warp per tile with the reference's per-tile stream; dspp = numSppForDenoising.
 cudaError_t LaunchAov(const DevScene& S, const DevCamera& C, const DevSettings& st, int aov,
                       int dspp, float* film, int* stackScratch, int* status, int tileBegin,
                       int tileEnd, cudaStream_t stream);
