@@ -449,6 +449,7 @@ __global__ void RaygenKernel(const DevJob* __restrict__ jobs, const WaveUnit* __
         wb.counts[2] = wb.counts[4] = wb.counts[5] = wb.counts[6] = 0;
         wb.counts[8] = wb.counts[9] = wb.counts[10] = 0;  // raster work list (64-bit) and overflow
         wb.counts[11] = wb.counts[12] = 0;                 // raster retrace list and its fetch
+        wb.counts[13] = 0;                                 // tail blocks finished
     }
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < kSortBins; k += gridDim.x * blockDim.x)
         wb.sortBins[k] = 0;  // ray-sort counts start at zero in every wave
@@ -923,21 +924,39 @@ struct TailSink {
 // queue and runs its closest hit, shade and next-event ray, bounce after bounce, until
 // the path ends or the wave's iterations are used up, exactly as the staged kernels
 // would (same functions, same per-path random stream, same order of radiance adds).
-// Late bounces hold few rays, and one launch spares each of them a sweep of three
-// latency-bound launches.
+// Bound by the latency of the longest path, where the staged kernels wait for the longest
+// ray of every stage and pay for three launches a bounce. With many paths the staged
+// kernels win: they refill their lanes and keep more warps resident. It runs
+//  - a whole wave of at most kTailWavePaths paths (RunWave). A 128x72 1-spp frame of 20,000
+//    triangles took 344 us staged and 185 us so; 147,456 paths 532 and 317 us; 65,536 paths
+//    in a Cornell box with an area light 502 and 331 us; 589,824 paths 663 and 643 us, but
+//    524,288 paths in the Cornell box 767 and 1102 us;
+//  - what is left of a wave from bounces 6, 9 or 12 on, if at most kTailPaths paths are
+//    (n <= most; otherwise the launch does nothing): a 640x360 8-spp frame over 400,000
+//    triangles 1980 -> 1819 us, a 2.2M-triangle 4K terrain frame 27.50 -> 27.00 ms;
+//  - what is left of a queue-polled wave once at most kTailPaths paths are: a 256x256 16-spp
+//    Cornell frame 1755 -> 1077 us (16,384 paths 1183 us, 262,144 paths 1140 us);
+//  - the bounces from WaveTuning::tailBounce on.
+constexpr int kTailWavePaths = 200000;
+constexpr int kTailPaths = 65536;
+constexpr int kTailBlocksPerSm = 4;  // 8 blocks: within 5% either way
 template <int kInteg>
 __global__ void __launch_bounds__(128) TailKernel(const DevJob* __restrict__ jobs, WaveBuffers wb,
-                                                  int cur, int iters) {
+                                                  int cur, int iters, int most) {
     __shared__ int2 sEnt[kSmemStack > 0 ? kSmemStack * kTraceBlock : 1];
     TravStack stk;
     stk.ent = sEnt;
     stk.code = nullptr;  // closest-hit and runtime any-hit visits only (Push / Pop)
     stk.sp = 0;
     const int n = wb.counts[cur];
+    if (n > most) return;
     const int sole = wb.desc->soleJob;
     int err = 0;
-    for (;;) {
-        const int i = atomicAdd(wb.counts + 4, 1);  // reset by the shade before
+    // few paths are spread over all the warps, as TraceQueue spreads a short queue
+    const int warps = gridDim.x * kTraceWarps;
+    const bool works = (int)(threadIdx.x & 31) < (n + warps - 1) / warps;
+    while (works) {
+        const int i = atomicAdd(wb.counts + 4, 1);  // reset by raygen or the shade before
         if (i >= n) break;
         const float4 ra = wb.ray[cur][2 * i], rb = wb.ray[cur][2 * i + 1];
         const int path = __float_as_int(ra.w);
@@ -984,6 +1003,16 @@ __global__ void __launch_bounds__(128) TailKernel(const DevJob* __restrict__ job
         }
     }
     if (err) atomicOr(wb.counts + 3, err);
+    // the last block to finish empties the queue for the stages that may follow
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(wb.counts + 13, 1) == (int)gridDim.x - 1) {
+            wb.counts[cur] = 0;
+            wb.counts[4] = 0;
+            wb.counts[13] = 0;
+        }
+    }
 }
 
 // It may run beside the next bounce's extend kernel (which touches neither the
@@ -1374,12 +1403,24 @@ struct StageOverlap {
     }
 };
 
-// tailFrom > 0: bounces from it0 + tailFrom on run in one TailKernel launch.
+static void LaunchTail(const DevJob* jobs, const WaveBuffers& wb, int integrator, int cur, int iters,
+                       int most, cudaStream_t stream) {
+    const int grid = SmCount() * kTailBlocksPerSm;
+    if (integrator == kPathTracing)
+        TailKernel<kPathTracing><<<grid, kTraceBlock, 0, stream>>>(jobs, wb, cur, iters, most);
+    else if (integrator == kSimplePathTracing)
+        TailKernel<kSimplePathTracing><<<grid, kTraceBlock, 0, stream>>>(jobs, wb, cur, iters, most);
+    else
+        TailKernel<-1><<<grid, kTraceBlock, 0, stream>>>(jobs, wb, cur, iters, most);
+}
+
+// tailFrom >= 0: bounces from it0 + tailFrom on run in one TailKernel launch. mayTail: the
+// wave may end in one earlier, where few paths are left.
 // envOnly: no job of the wave has area lights (the any-hit shadow kernel).
 static void LaunchBounces(const DevJob* jobs, const WaveUnit* units, const WaveBuffers& wb,
                           int integrator, int grid, int it0, int count, cudaStream_t stream,
                           WaveProfile* prof, int* nl, bool sort, StageOverlap* ov, bool envOnly,
-                          int tailFrom = 0, bool raster = false) {
+                          int tailFrom = -1, bool raster = false, bool mayTail = false) {
     StageEvents* ev = prof ? (StageEvents*)prof->events : nullptr;
     const int block = kTraceBlock;
     const int sgrid = ShadeGrid(grid);
@@ -1387,20 +1428,16 @@ static void LaunchBounces(const DevJob* jobs, const WaveUnit* units, const WaveB
     for (int it = it0; it < it0 + count; it++) {
         // sorted bounces trace queue 0 and reorder the rays shade appends to queue 1 back into it
         const int cur = sort ? 0 : (it & 1);
-        if (tailFrom > 0 && it - it0 == tailFrom) {
+        const int at = it - it0;
+        const bool all = at == tailFrom;
+        if (all || (mayTail && (at == 6 || at == 9 || at == 12))) {
             if (pendingShadow) {  // the tail adds radiance the pending shadow stage also adds to
                 cudaStreamWaitEvent(stream, ov->join, 0);
                 pendingShadow = false;
             }
-            const int left = it0 + count - it;
-            if (integrator == kPathTracing)
-                TailKernel<kPathTracing><<<grid, block, 0, stream>>>(jobs, wb, cur, left);
-            else if (integrator == kSimplePathTracing)
-                TailKernel<kSimplePathTracing><<<grid, block, 0, stream>>>(jobs, wb, cur, left);
-            else
-                TailKernel<-1><<<grid, block, 0, stream>>>(jobs, wb, cur, left);
+            LaunchTail(jobs, wb, integrator, cur, it0 + count - it, all ? INT_MAX : kTailPaths, stream);
             *nl += 1;
-            break;
+            if (all) break;
         }
         if (ev) ev->Begin(1, stream);
         if (it == 0 && raster) {  // the traced units' paths, then the rasterised ones
@@ -1443,7 +1480,9 @@ static void LaunchBounces(const DevJob* jobs, const WaveUnit* units, const WaveB
             TallyKernel<<<1, 1, 0, stream>>>(wb.counts, cur, prof->devCounters);
             ev->Begin(3, stream);
         }
-        if (ov) {
+        if (integrator == kSimplePathTracing) {
+            // no next-event rays
+        } else if (ov) {
             cudaEventRecord(ov->fork, stream);
             cudaStreamWaitEvent(ov->side, ov->fork, 0);
             if (envOnly) ShadowKernel<true><<<grid, block, 0, ov->side>>>(jobs, wb);
@@ -1456,7 +1495,7 @@ static void LaunchBounces(const DevJob* jobs, const WaveUnit* units, const WaveB
             ShadowKernel<false><<<grid, block, 0, stream>>>(jobs, wb);
         }
         if (ev) ev->End(3, stream);
-        *nl += 3;
+        *nl += integrator == kSimplePathTracing ? 2 : 3;
         if (sort) {
             SortKeysKernel<<<grid, block, 0, stream>>>(jobs, wb, 1);
             SortScanKernel<<<1, 1024, 0, stream>>>(wb);
@@ -1590,7 +1629,9 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
     d.soleJob = shape.soleJob;
     d.band = tune.band > 0 ? tune.band : 8;
     // the first bounce rasterised where the wave allows it (raster_primary.cuh)
-    const bool raster = shape.raster > 0 && tune.primaryTraversal != 1 && tune.sortRays == 0 &&
+    const bool sort = tune.sortRays != 0;
+    const bool whole = !prof && !sort && shape.nPaths <= kTailWavePaths;
+    const bool raster = !whole && shape.raster > 0 && tune.primaryTraversal != 1 && tune.sortRays == 0 &&
                         shape.iters >= 0;
     d.rasterFrom = raster ? shape.rasterFrom : shape.nPaths;
     d.rasterUnit0 = raster ? shape.rasterUnit0 : shape.nUnits;
@@ -1599,10 +1640,10 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
     cudaError_t e = cudaMemcpyAsync(wb.desc, &d, sizeof(d), cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) return e;
     int nl = 0;
-    const bool sort = tune.sortRays != 0;
     // the last bounces in one launch (fixed-depth waves; profiled renders keep every stage)
-    const int tailFrom = (!prof && !sort && tune.tailBounce > 0 && shape.iters > tune.tailBounce)
-                           ? tune.tailBounce : 0;
+    const int tailFrom = whole ? 0
+                         : (!prof && !sort && tune.tailBounce > 0 && shape.iters > tune.tailBounce)
+                           ? tune.tailBounce : -1;
     // shadow stages beside the next extend, on the owner's side stream (not when profiling,
     // whose stage timers need one stream)
     StageOverlap* ov =
@@ -1610,11 +1651,12 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
     const bool envOnly = !shape.areaLights;
     const WaveGraphKey key{jobs, units, wb.ray[0], wb.capacity, shape.iters, shape.integrator, grid,
                            sort ? 1 : 0, accumulate ? 1 : 0, tailFrom, raster ? 1 : 0, envOnly ? 1 : 0};
-    if (shape.iters >= 0) {
+    if (shape.iters >= 0 || whole) {
+        const int iters = shape.iters >= 0 ? shape.iters : kMaxReplayBounces;
         auto record = [&](int* n) {
             RaygenKernel<<<grid, block, 0, stream>>>(jobs, units, wb, 0, raster ? 1 : 0);
-            LaunchBounces(jobs, units, wb, shape.integrator, grid, 0, shape.iters, stream, prof, n, sort,
-                          ov, envOnly, tailFrom, raster);
+            LaunchBounces(jobs, units, wb, shape.integrator, grid, 0, iters, stream, prof, n, sort,
+                          ov, envOnly, tailFrom, raster, !sort);
             if (accumulate) AccumulateKernel<<<grid, block, 0, stream>>>(jobs, units, wb);
             *n += accumulate ? 2 : 1;
         };
@@ -1624,8 +1666,8 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
             if (ev) ev->Begin(0, stream);
             RaygenKernel<<<grid, block, 0, stream>>>(jobs, units, wb, 0, raster ? 1 : 0);
             if (ev) ev->End(0, stream);
-            LaunchBounces(jobs, units, wb, shape.integrator, grid, 0, shape.iters, stream, prof, &nl, sort,
-                          ov, envOnly, tailFrom, raster);
+            LaunchBounces(jobs, units, wb, shape.integrator, grid, 0, iters, stream, prof, &nl, sort,
+                          ov, envOnly, tailFrom, raster, !sort && !prof);
             if (accumulate) {
                 if (ev) ev->Begin(4, stream);
                 AccumulateKernel<<<grid, block, 0, stream>>>(jobs, units, wb);
@@ -1645,6 +1687,11 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
                 e = cudaMemcpyAsync(wb.hostCount, wb.counts, sizeof(int), cudaMemcpyDeviceToHost, stream);
                 if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
                 if (e != cudaSuccess || *wb.hostCount == 0 || it >= kMaxReplayBounces) break;
+                if (!prof && !sort && *wb.hostCount <= kTailPaths) {
+                    LaunchTail(jobs, wb, shape.integrator, 0, kMaxReplayBounces - it, INT_MAX, stream);
+                    nl++;
+                    break;
+                }
             }
             if (useGraphs) {
                 WaveGraphKey k = key;
