@@ -329,21 +329,37 @@ __device__ __noinline__ void ResolveTie(const DevScene* S, V3 o, V3 d, float tmi
     ResolveTieInline(S, o, d, tmin, tmax, best, tBest);
 }
 
+// Lanes of a warp that take entries of a queue of n: a short queue is spread over
+// kSpreadWarps warps per SM instead of filling few. Fewer rays a warp diverge less, and a
+// launch lasts as long as its slowest warp: a 128x72 1-spp frame of nine such queues took
+// 356 us spread over all warps against 478 with full ones. But beyond what keeps an SM
+// busy, more warps with fewer lanes only issue more instructions: a Cornell frame of
+// 427,180 paths and 4 bounces took 212 us unspread and 202, 202, 217 and 242 us with 4, 8, 16
+// and 28 warps per SM; a 512x288 4-spp frame of 20,000 triangles 869 us unspread, 650, 645,
+// 650 and 666 us.
+constexpr int kSpreadWarps = 6;
+__device__ __forceinline__ int LanesUsed(int n) {
+    unsigned sms;
+    asm("mov.u32 %0, %%nsmid;" : "=r"(sms));
+    const int warps = (int)sms * kSpreadWarps;
+    return min(32, max(1, (n + warps - 1) / warps));
+}
+
 // Q provides: void Load(int i, LaneRay&) (ray, range, and the scene: nodes = nullptr
 // for an empty scene) and void Finish(int i, const LaneRay&).
 // Must be called by every lane of the warp, in blocks of kTraceBlock threads.
 // kAnyHit: every ray Q loads is an any-hit ray.
-template <bool kAnyHit, class Q>
+// kFixedShare: each warp takes its share of a short queue by its index instead of from the
+// counter. Two round trips to the counter fewer: 22.3 -> 21.4 us for 1000 rays, 37.5 -> 36.0
+// us for 4000; in the wave's trace kernels the extra code costs registers (an interior
+// frame 4.28 -> 4.44 ms), so only the ray queries use it.
+template <bool kAnyHit, bool kFixedShare = false, class Q>
 __device__ void TraceQueue(Q& q, int n, int* fetch, int& err) {
     __shared__ int2 sEnt[!kAnyHit && kSmemStack > 0 ? kSmemStack * kTraceBlock : 1];
     __shared__ int sCode[kAnyHit && kSmemStack > 0 ? kSmemStack * kTraceBlock : 1];
     const int lane = threadIdx.x & 31;
     const unsigned lowerLanes = (1u << lane) - 1u;
-    const int warps = gridDim.x * kTraceWarps;
-    // A queue shorter than the grid's lanes is spread over all its warps: fewer rays a warp
-    // diverge less, and the launch lasts as long as its slowest warp. A 128x72 1-spp frame of
-    // nine such queues took 356 us against 478 with full warps.
-    const int lim = min(32, max(1, (n + warps - 1) / warps));
+    const int lim = LanesUsed(n);
     LaneRay r;
     int idx = -1;
     bool active = false;
@@ -359,9 +375,14 @@ __device__ void TraceQueue(Q& q, int n, int* fetch, int& err) {
         if (!exhausted && 32 - nIdle <= (3 * lim) / 4) {
             const int take = min(nIdle, lim - (32 - nIdle));
             int first = 0;
-            if (lane == 0) first = atomicAdd(fetch, take);
-            first = __shfl_sync(kFullMask, first, 0);
-            exhausted = first + take >= n;
+            if (kFixedShare && lim <= 16) {
+                first = (blockIdx.x * kTraceWarps + (threadIdx.x >> 5)) * lim;
+                exhausted = true;
+            } else {
+                if (lane == 0) first = atomicAdd(fetch, take);
+                first = __shfl_sync(kFullMask, first, 0);
+                exhausted = first + take >= n;
+            }
             const int k = __popc(idle & lowerLanes);
             if (!active && k < take && first + k < n) {
                 idx = first + k;
@@ -952,7 +973,8 @@ __global__ void __launch_bounds__(128) TailKernel(const DevJob* __restrict__ job
     if (n > most) return;
     const int sole = wb.desc->soleJob;
     int err = 0;
-    // few paths are spread over all the warps, as TraceQueue spreads a short queue
+    // few paths are spread over all the warps (128x72 1-spp frame: 190 us, over half or a
+    // quarter of them 218 and 224 us)
     const int warps = gridDim.x * kTraceWarps;
     const bool works = (int)(threadIdx.x & 31) < (n + warps - 1) / warps;
     while (works) {
@@ -1122,7 +1144,7 @@ __global__ void __launch_bounds__(128) TraceKernel(DevScene S, int n, const floa
     RayBatchQueue q{&S, S.numWide > 0 ? S.wide : nullptr, S.tris, S.numWide, S.numTris, rays, tmin,
                     tmax, triOut, distOut};
     int err = 0;
-    TraceQueue<false>(q, n, fetch, err);
+    TraceQueue<false, true>(q, n, fetch, err);
 }
 
 // Profiling helpers: ray tallies and the reference traversal's work per ray.
