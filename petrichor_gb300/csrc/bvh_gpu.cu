@@ -16,7 +16,9 @@
 //    key <= p counting down. The scans swap the pairs (L_k, R_k) for k < K, where K is
 //    the first k with L_k >= R_k (a missing L_k counts as +inf), and return the cut
 //    min(L_K, R_{K-1}): a swapped-in element at R_{K-1} stops the final left scan.
-//    Positions and ranks come from one prefix sum of the two flags.
+//    Positions and ranks come from one prefix sum of the two flags. Rounds over all of
+//    global memory only run for subranges of more than BlockSortMax(2) elements; a smaller one
+//    is partitioned to its end by one block in shared memory (BlockSortKernel).
 //  - Bin assignment, bin bounds and the 16-candidate SAH cost use the reference's float
 //    expressions (no contraction: the file is built with -fmad=false).
 //  - Node bounds are std::min/std::max merges in range order: among equal extremes
@@ -30,6 +32,7 @@
 // build reports failure instead of returning a tree.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <climits>
 #include <cstddef>
@@ -243,13 +246,35 @@ struct Counters {  // device words
     int small;      // insertion blocks
     int heap;       // heapsort subranges
     int error;
-    int pad[2];
+    int largest;    // most primitives of an active node of the next level
+    int block[3];   // subranges for the block sorts, by size class
 };
+
+// Size classes of the block sorts: a subrange of at most BlockSortMax(c) elements is sorted by
+// one block of BlockSortMax(c) / BlockSortItems(c) threads.
+__host__ __device__ constexpr int BlockSortMax(int c) { return c == 0 ? 128 : c == 1 ? 1024 : 8192; }
+__host__ __device__ constexpr int BlockSortItems(int c) { return c == 0 ? 4 : 8; }
+struct BlockLists {
+    int4* list[3];  // {first, last, depth budget, 0}
+    int cap[3];
+};
+// Hands the subrange [first, last) of more than kSmallSort elements to the block sorts;
+// false when it is too large for them.
+__device__ __forceinline__ bool PushBlockRange(const BlockLists& bl, Counters* cnt, int first, int last, int depth) {
+    const int n = last - first;
+    if (n > BlockSortMax(2)) return false;
+    const int c = n <= BlockSortMax(0) ? 0 : n <= BlockSortMax(1) ? 1 : 2;
+    const int x = atomicAdd(&cnt->block[c], 1);
+    if (x < bl.cap[c]) bl.list[c][x] = make_int4(first, last, depth, 0);
+    else atomicOr(&cnt->error, kErrCapacity);
+    return true;
+}
 
 __global__ void NodeAxisKernel(int nActive, LevelNodes nodes, const uint32_t* __restrict__ cb,
                                int* __restrict__ axis, float* __restrict__ cbLo,
                                float* __restrict__ len, int* __restrict__ segOfNode, SegList segs,
-                               int2* __restrict__ small, Counters* cnt, int segCap, int smallCap) {
+                               int2* __restrict__ small, BlockLists bl, Counters* cnt, int segCap,
+                               int smallCap) {
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= nActive) return;
     float lo[3], hi[3];
@@ -269,6 +294,7 @@ __global__ void NodeAxisKernel(int nActive, LevelNodes nodes, const uint32_t* __
     const int b = nodes.begin[a], e = nodes.end[a], n = e - b;
     segOfNode[a] = -1;
     if (n > kSmallSort) {
+        if (PushBlockRange(bl, cnt, b, e, 2 * FloorLog2(n))) return;
         const int s = atomicAdd(&cnt->segs, 1);
         if (s >= segCap) {
             atomicOr(&cnt->error, kErrCapacity);
@@ -313,26 +339,21 @@ __device__ __forceinline__ void SwapAt(float* key, int* ids, int x, int y) {
     ids[y] = d;
 }
 
+// std::__move_median_to_first(first, first + 1, mid, last - 1): the pivot's place.
+__device__ __forceinline__ int MedianPlace(const float* key, int f, int l) {
+    const int a = f + 1, b = f + (l - f) / 2, c = l - 1;
+    const float ka = key[a], kb = key[b], kc = key[c];
+    if (ka < kb) return kb < kc ? b : ka < kc ? c : a;
+    return ka < kc ? a : kb < kc ? c : b;
+}
+
 // __unguarded_partition_pivot's pivot: std::__move_median_to_first(first, first + 1,
 // mid, last - 1).
 __global__ void PivotKernel(int nSeg, SegList segs, float* __restrict__ key, int* __restrict__ ids) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nSeg) return;
     const int f = segs.first[s], l = segs.last[s];
-    const int a = f + 1, b = f + (l - f) / 2, c = l - 1;
-    const float ka = key[a], kb = key[b], kc = key[c];
-    int m;
-    if (ka < kb) {
-        if (kb < kc) m = b;
-        else if (ka < kc) m = c;
-        else m = a;
-    } else if (ka < kc) {
-        m = a;
-    } else if (kb < kc) {
-        m = c;
-    } else {
-        m = b;
-    }
+    const int m = MedianPlace(key, f, l);
     SwapAt(key, ids, f, m);
     segs.pivot[s] = key[f];
     segs.K[s] = INT_MAX;
@@ -413,8 +434,8 @@ __global__ void SwapKernel(int T, const int* __restrict__ seg, SegList segs,
 // both halves with the decremented depth; more than 16 elements and no depth left:
 // heapsort; 16 or fewer: left to the final insertion sort.
 __global__ void SplitSegsKernel(int nSeg, SegList segs, SegList next, int2* __restrict__ small,
-                                int2* __restrict__ heap, Counters* cnt, int segCap, int smallCap,
-                                int heapCap) {
+                                int2* __restrict__ heap, BlockLists bl, Counters* cnt, int segCap,
+                                int smallCap, int heapCap) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nSeg) return;
     const int f = segs.first[s], l = segs.last[s], cut = segs.cut[s];
@@ -428,7 +449,7 @@ __global__ void SplitSegsKernel(int nSeg, SegList segs, SegList next, int2* __re
                 const int h = atomicAdd(&cnt->heap, 1);
                 if (h < heapCap) heap[h] = make_int2(lo[c], hi[c]);
                 else atomicOr(&cnt->error, kErrCapacity);
-            } else {
+            } else if (!PushBlockRange(bl, cnt, lo[c], hi[c], d)) {
                 const int x = atomicAdd(&cnt->segs, 1);
                 if (x < segCap) {
                     next.first[x] = lo[c];
@@ -486,10 +507,8 @@ __device__ void AdjustHeap(float* key, int* ids, int first, int hole, int len, f
     ids[first + hole] = vi;
 }
 
-__global__ void HeapSortKernel(int nHeap, const int2* __restrict__ heap, float* key, int* ids) {
-    const int h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= nHeap) return;
-    const int first = heap[h].x, last = heap[h].y, len = last - first;
+__device__ void HeapSortRange(float* key, int* ids, int first, int last) {
+    const int len = last - first;
     if (len < 2) return;
     for (int parent = (len - 2) / 2;; parent--) {  // __make_heap
         AdjustHeap(key, ids, first, parent, len, key[first + parent], ids[first + parent]);
@@ -505,11 +524,14 @@ __global__ void HeapSortKernel(int nHeap, const int2* __restrict__ heap, float* 
     }
 }
 
+__global__ void HeapSortKernel(const Counters* cnt, int heapCap, const int2* __restrict__ heap, float* key, int* ids) {
+    const int n = min(cnt->heap, heapCap);
+    for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < n; h += gridDim.x * blockDim.x)
+        HeapSortRange(key, ids, heap[h].x, heap[h].y);
+}
+
 // The final insertion sort on one block the partitioning left (stable, <= 16 elements).
-__global__ void InsertionKernel(int nSmall, const int2* __restrict__ small, float* key, int* ids) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nSmall) return;
-    const int first = small[b].x, last = small[b].y;
+__device__ __forceinline__ void InsertionRange(float* key, int* ids, int first, int last) {
     for (int i = first + 1; i < last; i++) {
         const float vk = key[i];
         const int vi = ids[i];
@@ -521,6 +543,206 @@ __global__ void InsertionKernel(int nSmall, const int2* __restrict__ small, floa
         }
         key[j] = vk;
         ids[j] = vi;
+    }
+}
+__global__ void InsertionKernel(const Counters* cnt, int smallCap, const int2* __restrict__ small, float* key, int* ids) {
+    const int n = min(cnt->small, smallCap);
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < n; b += gridDim.x * blockDim.x)
+        InsertionRange(key, ids, small[b].x, small[b].y);
+}
+
+// The introsort of one subrange of at most kN elements by one block, in shared memory: the
+// same rounds as the kernels over global memory below (median to the front, flags, prefix
+// sum, ranks, swaps, split), then the insertion sorts of its leftovers. A subrange whose
+// depth budget runs out goes to the heapsort list.
+// Bound by the latency of seven barriers a round (157 us for ranges of up to 8192). It took
+// the place of rounds over all primitives that each ended in a read of the counters by the
+// host, 68 us a round: 400,000 triangles took 309 of them and 24.6 ms, now 49 and 10.7 ms;
+// 20,000 triangles 144 and 9.9 ms, now 3 and 2.8 ms; 1.0M triangles 34.2 -> 16.3 ms.
+template <int kN, int kItems>
+struct BlockSortShared {
+    static constexpr int kThreadsB = kN / kItems;
+    static constexpr int kSegs = kN / (kSmallSort + 1) + 1;
+    float key[kN];
+    int id[kN];
+    uint32_t pre[kN + 1];  // exclusive counts of the flags: left stops low, right stops high
+    uint16_t lpos[kN], rpos[kN];
+    int16_t seg[kN];       // open subrange of each position, -1: none
+    uint16_t small[kN / 2], smallLen[kN / 2];
+    uint16_t first[2][kSegs], last[2][kSegs];
+    int16_t depth[2][kSegs];
+    float pivot[kSegs];
+    int K[kSegs], cut[kSegs];
+    int16_t newL[kSegs], newR[kSegs];
+    uint32_t warpSum[kThreadsB / 32];
+    int nSeg[2], nSmall;
+};
+template <int kN, int kItems>
+__global__ void __launch_bounds__(kN / kItems) BlockSortKernel(const int* __restrict__ count, int cap,
+                                                               const int4* __restrict__ list, float* __restrict__ key,
+                                                               int* __restrict__ ids, int2* __restrict__ heap,
+                                                               Counters* cnt, int heapCap) {
+    using Shared = BlockSortShared<kN, kItems>;
+    constexpr int kT = Shared::kThreadsB;
+    extern __shared__ __align__(16) char raw[];
+    Shared& m = *reinterpret_cast<Shared*>(raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t below = (1u << lane) - 1u;
+    const int total = min(*count, cap);
+    for (int r = blockIdx.x; r < total; r += gridDim.x) {
+        const int4 range = list[r];
+        const int base = range.x, n = range.y - range.x;
+        __syncthreads();  // the previous subrange is written back
+        for (int i = tid; i < n; i += kT) {
+            m.key[i] = key[base + i];
+            m.id[i] = ids[base + i];
+            m.seg[i] = 0;
+        }
+        for (int i = n + tid; i < kN; i += kT) m.seg[i] = -1;
+        if (tid == 0) {
+            m.first[0][0] = 0;
+            m.last[0][0] = (uint16_t)n;
+            m.depth[0][0] = (int16_t)range.z;
+            m.nSeg[0] = 1;
+            m.nSmall = 0;
+        }
+        __syncthreads();
+        int cur = 0;
+        // every round splits each open subrange into two shorter ones, and the depth
+        // budgets bound the rounds
+        while (m.nSeg[cur] > 0) {
+            const int nSeg = m.nSeg[cur], nxt = cur ^ 1;
+            for (int s = tid; s < nSeg; s += kT) {
+                const int f = m.first[cur][s];
+                SwapAt(m.key, m.id, f, MedianPlace(m.key, f, m.last[cur][s]));
+                m.pivot[s] = m.key[f];
+                m.K[s] = INT_MAX;
+            }
+            if (tid == 0) m.nSeg[nxt] = 0;
+            __syncthreads();
+            // flags and their prefix sums: a warp takes 32 * kItems consecutive positions
+            uint32_t bx[kItems], by[kItems], sum = 0;
+#pragma unroll
+            for (int j = 0; j < kItems; j++) {
+                const int i = (warp * kItems + j) * 32 + lane;
+                const int s = m.seg[i];
+                bool x = false, y = false;
+                if (s >= 0) {
+                    const float pv = m.pivot[s], k = m.key[i];
+                    x = i > m.first[cur][s] && !(k < pv);
+                    y = !(pv < k);
+                }
+                bx[j] = __ballot_sync(kFull, x);
+                by[j] = __ballot_sync(kFull, y);
+                sum += (uint32_t)__popc(bx[j]) | ((uint32_t)__popc(by[j]) << 16);
+            }
+            if (lane == 0) m.warpSum[warp] = sum;
+            __syncthreads();
+            uint32_t run = lane < warp ? m.warpSum[lane] : 0u;  // at most 32 warps
+            for (int d = 16; d >= 1; d >>= 1) run += __shfl_xor_sync(kFull, run, d);
+#pragma unroll
+            for (int j = 0; j < kItems; j++) {
+                const int i = (warp * kItems + j) * 32 + lane;
+                m.pre[i] = run + ((uint32_t)__popc(bx[j] & below) | ((uint32_t)__popc(by[j] & below) << 16));
+                run += (uint32_t)__popc(bx[j]) | ((uint32_t)__popc(by[j]) << 16);
+            }
+            if (tid == kT - 1) m.pre[kN] = run;
+            __syncthreads();
+            // ranks (RanksKernel)
+#pragma unroll
+            for (int j = 0; j < kItems; j++) {
+                const int i = (warp * kItems + j) * 32 + lane;
+                const int s = m.seg[i];
+                bool stops = false;
+                int k = 0;
+                if (s >= 0) {
+                    const int f = m.first[cur][s];
+                    const uint32_t pi = m.pre[i], pn = m.pre[i + 1], pl = m.pre[m.last[cur][s]];
+                    if ((pn ^ pi) & 0xffffu) {  // a left-scan stop: rank k counting up
+                        k = (int)(pi & 0xffffu) - (int)(m.pre[f + 1] & 0xffffu) + 1;
+                        m.lpos[f + k - 1] = (uint16_t)i;
+                        stops = (int)(pl >> 16) - (int)(pn >> 16) < k;  // right-scan stops above i
+                    }
+                    if ((pn >> 16) != (pi >> 16))  // a right-scan stop: rank counting down
+                        m.rpos[f + (int)(pl >> 16) - (int)(pi >> 16) - 1] = (uint16_t)i;
+                }
+                // the first stopping rank: of a warp's stops in one subrange, the lowest position's
+                const uint32_t all = __ballot_sync(kFull, stops);
+                const int before = __shfl_up_sync(kFull, s, 1);
+                const uint32_t starts = __ballot_sync(kFull, lane == 0 || s != before);
+                const int start = 31 - __clz(starts & (below | (1u << lane)));
+                if (stops && (all & below & ~((1u << start) - 1u)) == 0) atomicMin(&m.K[s], k);
+            }
+            __syncthreads();
+            // swaps (SwapKernel)
+#pragma unroll
+            for (int j = 0; j < kItems; j++) {
+                const int i = (warp * kItems + j) * 32 + lane;
+                const int s = m.seg[i];
+                if (s < 0) continue;
+                const int f = m.first[cur][s], l = m.last[cur][s], k = i - f + 1;
+                const int numL = (int)(m.pre[l] & 0xffffu) - (int)(m.pre[f + 1] & 0xffffu);
+                const int K = min(m.K[s], numL + 1);
+                if (k < K) {
+                    SwapAt(m.key, m.id, m.lpos[f + k - 1], m.rpos[f + k - 1]);
+                } else if (k == K) {
+                    int cut;
+                    if (K <= numL) cut = K >= 2 ? min(m.lpos[f + K - 1], m.rpos[f + K - 2]) : m.lpos[f];
+                    else if (K >= 2) cut = m.rpos[f + K - 2];
+                    else cut = -1;
+                    if (cut < 0) atomicOr(&cnt->error, kErrPartition);
+                    if (cut <= f || cut >= l) {
+                        atomicOr(&cnt->error, kErrCut);
+                        cut = f + 1;  // keeps the bookkeeping bounded; the build reports failure
+                    }
+                    m.cut[s] = cut;
+                }
+            }
+            __syncthreads();
+            // split (SplitSegsKernel)
+            for (int s = tid; s < nSeg; s += kT) {
+                const int cut = m.cut[s], d = m.depth[cur][s] - 1;
+                const int lo[2] = {m.first[cur][s], cut}, hi[2] = {cut, m.last[cur][s]};
+                int idx[2] = {-1, -1};
+                for (int c = 0; c < 2; c++) {
+                    const int len = hi[c] - lo[c];
+                    if (len > kSmallSort) {
+                        if (d == 0) {
+                            const int h = atomicAdd(&cnt->heap, 1);
+                            if (h < heapCap) heap[h] = make_int2(base + lo[c], base + hi[c]);
+                            else atomicOr(&cnt->error, kErrCapacity);
+                        } else {
+                            const int x = atomicAdd(&m.nSeg[nxt], 1);
+                            m.first[nxt][x] = (uint16_t)lo[c];
+                            m.last[nxt][x] = (uint16_t)hi[c];
+                            m.depth[nxt][x] = (int16_t)d;
+                            idx[c] = x;
+                        }
+                    } else if (len >= 2) {
+                        const int x = atomicAdd(&m.nSmall, 1);
+                        m.small[x] = (uint16_t)lo[c];
+                        m.smallLen[x] = (uint16_t)len;
+                    }
+                }
+                m.newL[s] = (int16_t)idx[0];
+                m.newR[s] = (int16_t)idx[1];
+            }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < kItems; j++) {
+                const int i = (warp * kItems + j) * 32 + lane;
+                const int s = m.seg[i];
+                if (s >= 0) m.seg[i] = i < m.cut[s] ? m.newL[s] : m.newR[s];
+            }
+            cur = nxt;
+            __syncthreads();
+        }
+        for (int b = tid; b < m.nSmall; b += kT) InsertionRange(m.key, m.id, m.small[b], m.small[b] + m.smallLen[b]);
+        __syncthreads();
+        for (int i = tid; i < n; i += kT) {
+            key[base + i] = m.key[i];
+            ids[base + i] = m.id[i];
+        }
     }
 }
 
@@ -723,12 +945,12 @@ __global__ void OrderedBoundsKernel(int T, int root, const int* __restrict__ nod
 }
 
 // The winning positions' own coordinates (their sign of zero included).
-__global__ void ResolveBoundsKernel(int nRecords, int recordBase, int T,
+__global__ void ResolveBoundsKernel(const Counters* cnt, int nodeCap, int recordBase, int T,
                                     const unsigned long long* __restrict__ acc,
                                     const int* __restrict__ ids, const float* __restrict__ box,
                                     float* __restrict__ out) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nRecords) return;
+    if (recordBase + r >= min(cnt->nodes, nodeCap)) return;
     for (int a = 0; a < 6; a++) {
         const unsigned long long k = acc[6 * (size_t)r + a];
         float v;
@@ -764,6 +986,7 @@ __global__ void NextLevelKernel(int nActive, const int* __restrict__ mid,
         next.begin[x] = tn.begin[r];
         next.end[x] = tn.end[r];
         childActive[2 * a + c] = x;
+        atomicMax(&cnt->largest, tn.end[r] - tn.begin[r]);
     }
 }
 
@@ -837,7 +1060,8 @@ __global__ void ResetCounters(Counters* c, int segs, int small, int heap, int ac
     if (segs) c->segs = 0;
     if (small) c->small = 0;
     if (heap) c->heap = 0;
-    if (active) c->active = 0;
+    if (active) c->active = c->largest = 0;
+    if (small) c->block[0] = c->block[1] = c->block[2] = 0;
 }
 
 // ---------------------------------------------------------------- host driver
@@ -855,6 +1079,20 @@ struct Arena {
         for (void* p : ptrs) cudaFree(p);
     }
 };
+
+// One size class of the block sorts, where a level's largest node reaches it.
+template <int kClass>
+int LaunchBlockSort(int largest, const BlockLists& bl, float* key, int* ids, int2* heap, Counters* cnt, int heapCap,
+                    cudaStream_t s) {
+    constexpr int kN = BlockSortMax(kClass), kItems = BlockSortItems(kClass);
+    if (largest <= (kClass == 0 ? kSmallSort : BlockSortMax(kClass - 1))) return 0;
+    const auto kernel = BlockSortKernel<kN, kItems>;
+    const int bytes = (int)sizeof(BlockSortShared<kN, kItems>);
+    if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    kernel<<<std::min(bl.cap[kClass], kClass == 2 ? 152 : kClass == 1 ? 1216 : 4864), kN / kItems, bytes, s>>>(
+      &cnt->block[kClass], bl.cap[kClass], bl.list[kClass], key, ids, heap, cnt, heapCap);
+    return 1;
+}
 
 }  // namespace
 
@@ -914,6 +1152,11 @@ cudaError_t BuildBinnedSahDevice(const float* positions, int numVertices, const 
                     ar.Get<int>(segCap), ar.Get<int>(segCap), ar.Get<int>(segCap), ar.Get<int>(segCap)};
     int2* small = ar.Get<int2>(smallCap);
     int2* heap = ar.Get<int2>(heapCap);
+    BlockLists bl;
+    for (int c = 0; c < 3; c++) {
+        bl.cap[c] = T / ((c == 0 ? kSmallSort : BlockSortMax(c - 1)) + 1) + 1;
+        bl.list[c] = ar.Get<int4>(bl.cap[c]);
+    }
     Counters* cnt = ar.Get<Counters>(1);
     int* ic = ar.Get<int>(nodeCap);
     int* index = ar.Get<int>(nodeCap);
@@ -964,6 +1207,8 @@ cudaError_t BuildBinnedSahDevice(const float* positions, int numVertices, const 
     cudaMemcpyAsync(dPos, positions, 3 * (size_t)numVertices * sizeof(float), cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dIdx, indices, 3 * t * sizeof(int32_t), cudaMemcpyHostToDevice, s);
     cudaMemsetAsync(cnt, 0, sizeof(Counters), s);
+    const int oneNode = 1;
+    cudaMemcpyAsync(&cnt->nodes, &oneNode, sizeof(int), cudaMemcpyHostToDevice, s);
     PrimKernel<<<Blocks(T), kThreads, 0, s>>>(dPos, dIdx, T, cent, box, ids);
     // the root record: all primitives in their input order
     {
@@ -976,13 +1221,11 @@ cudaError_t BuildBinnedSahDevice(const float* positions, int numVertices, const 
         cudaMemsetAsync(acc + 3, 0, 3 * sizeof(unsigned long long), s);
         OrderedBoundsKernel<<<Blocks(T, kThreads * kRun), kThreads, 0, s>>>(
           T, 1, nodeOf, mid, childBase, 0, ids, box, acc);
-        ResolveBoundsKernel<<<1, 32, 0, s>>>(1, 0, T, acc, ids, box, tn.box);
+        ResolveBoundsKernel<<<1, 32, 0, s>>>(cnt, nodeCap, 0, T, acc, ids, box, tn.box);
         launches += 3;
     }
-    const int oneNode = 1;
-    cudaMemcpyAsync(&cnt->nodes, &oneNode, sizeof(int), cudaMemcpyHostToDevice, s);
     std::vector<int> levelStart = {0, 1};
-    int nActive = 0;
+    int nActive = 0, largest = T;  // active nodes of the level, primitives of the largest
     if (T > kLeafMax) {
         const int rootRec[3] = {0, 0, T};
         cudaMemcpyAsync(lv[0].tempId, &rootRec[0], sizeof(int), cudaMemcpyHostToDevice, s);
@@ -1002,67 +1245,64 @@ cudaError_t BuildBinnedSahDevice(const float* positions, int numVertices, const 
         ResetCounters<<<1, 1, 0, s>>>(cnt, 1, 1, 1, 1);
         CentroidBoundsKernel<<<Blocks(T, kThreads * kRun), kThreads, 0, s>>>(T, nodeOf, ids, cent, cb);
         NodeAxisKernel<<<Blocks(nActive), kThreads, 0, s>>>(nActive, L, cb, axis, cbLo, len, segOfNode,
-                                                          sl[0], small, cnt, segCap, smallCap);
+                                                          sl[0], small, bl, cnt, segCap, smallCap);
         KeysKernel<<<Blocks(T), kThreads, 0, s>>>(T, nodeOf, ids, cent, axis, segOfNode, key, seg);
         launches += 5;
-        cudaError_t e = fetch();
-        if (e != cudaSuccess) return e;
-        int nSeg = hc->segs, sc = 0;
-        // std::sort of every node range: partition rounds over all open subranges
-        while (nSeg > 0 && hc->error == 0) {
-            rounds++;
-            SegList& S = sl[sc];
-            SegList& X = sl[sc ^ 1];
-            PivotKernel<<<Blocks(nSeg), kThreads, 0, s>>>(nSeg, S, key, ids);
-            FlagsKernel<<<Blocks(T + 1), kThreads, 0, s>>>(T, seg, S, key, flags);
-            ExclusiveScan(flags, pre, T + 1, scan, 0, s);
-            RanksKernel<<<Blocks(T), kThreads, 0, s>>>(T, seg, S, pre, lpos, rpos);
-            SwapKernel<<<Blocks(T), kThreads, 0, s>>>(T, seg, S, pre, lpos, rpos, key, ids, cnt);
-            ResetCounters<<<1, 1, 0, s>>>(cnt, 1, 0, 0, 0);
-            SplitSegsKernel<<<Blocks(nSeg), kThreads, 0, s>>>(nSeg, S, X, small, heap, cnt, segCap,
-                                                             smallCap, heapCap);
-            ResegKernel<<<Blocks(T), kThreads, 0, s>>>(T, seg, S);
-            launches += 8 + 2 * (int)scan.levels.size() + 1;
+        cudaError_t e = cudaSuccess;
+        // std::sort of every node range: partition rounds over all open subranges too large
+        // for one block, then the others a block each
+        if (largest > BlockSortMax(2)) {
             if ((e = fetch()) != cudaSuccess) return e;
-            nSeg = hc->segs;
-            sc ^= 1;
+            int nSeg = hc->segs, sc = 0;
+            while (nSeg > 0 && hc->error == 0) {
+                rounds++;
+                SegList& S = sl[sc];
+                SegList& X = sl[sc ^ 1];
+                PivotKernel<<<Blocks(nSeg), kThreads, 0, s>>>(nSeg, S, key, ids);
+                FlagsKernel<<<Blocks(T + 1), kThreads, 0, s>>>(T, seg, S, key, flags);
+                ExclusiveScan(flags, pre, T + 1, scan, 0, s);
+                RanksKernel<<<Blocks(T), kThreads, 0, s>>>(T, seg, S, pre, lpos, rpos);
+                SwapKernel<<<Blocks(T), kThreads, 0, s>>>(T, seg, S, pre, lpos, rpos, key, ids, cnt);
+                ResetCounters<<<1, 1, 0, s>>>(cnt, 1, 0, 0, 0);
+                SplitSegsKernel<<<Blocks(nSeg), kThreads, 0, s>>>(nSeg, S, X, small, heap, bl, cnt, segCap,
+                                                                 smallCap, heapCap);
+                ResegKernel<<<Blocks(T), kThreads, 0, s>>>(T, seg, S);
+                launches += 8 + 2 * (int)scan.levels.size() + 1;
+                if ((e = fetch()) != cudaSuccess) return e;
+                nSeg = hc->segs;
+                sc ^= 1;
+            }
+            if (hc->error) break;
         }
-        if (hc->error) break;
-        heapsorts += hc->heap;
-        if (hc->heap > 0) {
-            HeapSortKernel<<<Blocks(hc->heap, 64), 64, 0, s>>>(hc->heap, heap, key, ids);
-            launches++;
-        }
-        if (hc->small > 0) {
-            InsertionKernel<<<Blocks(hc->small), kThreads, 0, s>>>(hc->small, small, key, ids);
-            launches++;
-        }
+        launches += LaunchBlockSort<0>(largest, bl, key, ids, heap, cnt, heapCap, s);
+        launches += LaunchBlockSort<1>(largest, bl, key, ids, heap, cnt, heapCap, s);
+        launches += LaunchBlockSort<2>(largest, bl, key, ids, heap, cnt, heapCap, s);
+        HeapSortKernel<<<64, 64, 0, s>>>(cnt, heapCap, heap, key, ids);
+        InsertionKernel<<<std::min(Blocks(smallCap), 1024), kThreads, 0, s>>>(cnt, smallCap, small, key, ids);
         // bins and the SAH split of every active node
         InitCodes<<<Blocks((long long)nActive * kBins), kThreads, 0, s>>>(bins, nActive * kBins, 7);
         BinsKernel<<<Blocks(T, kThreads * kRun), kThreads, 0, s>>>(T, nodeOf, ids, key, cbLo, len, box, bins);
         SahKernel<<<Blocks(nActive), kThreads, 0, s>>>(nActive, L, bins, tn, mid, childBase, cnt, nodeCap);
-        launches += 3;
-        if ((e = fetch()) != cudaSuccess) return e;
-        if (hc->error) break;
-        const int recordBase = nodesTotal, nRecords = hc->nodes - recordBase;
-        nodesTotal = hc->nodes;
-        if (nRecords > 0) {
-            InitBounds64<<<Blocks(nRecords), kThreads, 0, s>>>(acc, nRecords);
-            OrderedBoundsKernel<<<Blocks(T, kThreads * kRun), kThreads, 0, s>>>(
-              T, 0, nodeOf, mid, childBase, recordBase, ids, box, acc);
-            ResolveBoundsKernel<<<Blocks(nRecords), kThreads, 0, s>>>(nRecords, recordBase, T, acc, ids,
+        // bounds of the new records (at most two a node)
+        const int recordBase = nodesTotal;
+        InitBounds64<<<Blocks(2 * nActive), kThreads, 0, s>>>(acc, 2 * nActive);
+        OrderedBoundsKernel<<<Blocks(T, kThreads * kRun), kThreads, 0, s>>>(
+          T, 0, nodeOf, mid, childBase, recordBase, ids, box, acc);
+        ResolveBoundsKernel<<<Blocks(2 * nActive), kThreads, 0, s>>>(cnt, nodeCap, recordBase, T, acc, ids,
                                                                    box, tn.box);
-            levelStart.push_back(nodesTotal);
-            launches += 3;
-        }
+        launches += 8;
         ResetCounters<<<1, 1, 0, s>>>(cnt, 0, 0, 0, 1);
         NextLevelKernel<<<Blocks(nActive), kThreads, 0, s>>>(nActive, mid, childBase, tn, N, childActive,
                                                            cnt, activeCap);
         NodeOfKernel<<<Blocks(T), kThreads, 0, s>>>(T, nodeOf, mid, childActive);
         launches += 3;
         if ((e = fetch()) != cudaSuccess) return e;
+        heapsorts += hc->heap;
         if (hc->error) break;
+        if (hc->nodes > nodesTotal) levelStart.push_back(hc->nodes);
+        nodesTotal = hc->nodes;
         nActive = hc->active;
+        largest = hc->largest;
         cur ^= 1;
     }
     if (hc->error) {
