@@ -27,15 +27,14 @@
 namespace ptg {
 
 // Minimum resident blocks per SM requested from the register allocator for the
-// trace (extend/shadow) and shade stages; 1 leaves the choice to the compiler. Trace: 7
-// blocks of 72 registers; 8 of 64 (which spill), 6 and 5 measured 17.65, 17.30 and 17.85 ms
-// against 16.90 for the closest hits of the 1.0M-triangle 1080p frame.
+// trace (extend/shadow) stages: 7 blocks of 72 registers; 8 of 64 (which spill), 6 and 5
+// measured 17.65, 17.30 and 17.85 ms against 16.90 for the closest hits of the
+// 1.0M-triangle 1080p frame.
 #ifndef PT_TRACE_MIN_BLOCKS
 #define PT_TRACE_MIN_BLOCKS 7
 #endif
-#ifndef PT_SHADE_MIN_BLOCKS
-#define PT_SHADE_MIN_BLOCKS 1
-#endif
+// Resident blocks per SM of the shade stage, and its grid (see ShadeKernel).
+constexpr int kShadeBlocks = 5;
 
 enum : int { kFlagNoSignCheck = 1 };
 enum : int { kShadowEnv = 0, kShadowArea = 1 };
@@ -554,48 +553,32 @@ __global__ void __launch_bounds__(128, PT_TRACE_MIN_BLOCKS) ExtendKernel(const D
 
 // kInteg: the integrator of every job in the wave, or -1 when the wave mixes them
 // (then read per path). A fixed integrator halves the kernel's code.
-// The staged shade kernel's sink: next-event entries and continuation rays go to the
-// queues (warp-aggregated appends), terminated paths add their radiance.
+// The staged shade kernel's sink: the next-event entry waits in shared memory and the
+// outcome in registers until the whole warp has shaded, so both appends share one round trip
+// to the counters.
 struct StageSink {
-    WaveBuffers& wb;
-    int nxt, path;
-    PathRng* rng;
-    __device__ __forceinline__ void Shadow(bool shadow, float4 sh0, float4 sh1, float4 sh2, float4 sh3) {
-        int sslot = WarpAppend(wb.counts + 2, shadow);
-#if PT_CHECK
-        if (shadow && sslot >= wb.capacity) {
-            atomicOr(wb.counts + 3, kErrBounds);
-            shadow = false;
-        }
-#endif
-        if (shadow) {
-            float4* e = wb.shadow + 4 * (size_t)sslot;
-            e[0] = sh0;
-            e[1] = sh1;
-            e[2] = sh2;
-            e[3] = sh3;
+    float4* sh;  // shared: the thread's next-event entry, kTraceBlock apart
+    bool shadow = false, cont = false;
+    Ray out;
+    float lastPdf = 0.0f, lastSin = 0.0f;
+    int flags = 0;
+    V3 L;
+    __device__ __forceinline__ void Shadow(bool s, float4 a, float4 b, float4 c, float4 d) {
+        shadow = s;
+        if (s) {
+            sh[0] = a;
+            sh[kTraceBlock] = b;
+            sh[2 * kTraceBlock] = c;
+            sh[3 * kTraceBlock] = d;
         }
     }
-    __device__ __forceinline__ void Done(bool cont, const Ray& out, float lastPdf, float lastSin,
-                                         int flags, V3 L) {
-        int rslot = WarpAppend(wb.counts + nxt, cont);
-#if PT_CHECK
-        if (cont && rslot >= wb.capacity) {
-            atomicOr(wb.counts + 3, kErrBounds);
-            cont = false;
-        }
-#endif
-        if (cont) {
-            wb.ray[nxt][2 * rslot] = make_float4(out.o.x, out.o.y, out.o.z, __int_as_float(path));
-            wb.ray[nxt][2 * rslot + 1] = make_float4(out.d.x, out.d.y, out.d.z, out.ior);
-            wb.qs0[nxt][rslot] = make_float4(out.T.x, out.T.y, out.T.z, out.prob);
-            wb.qs1[nxt][rslot] = make_float4(lastPdf, lastSin, __int_as_float(out.bounce),
-                                             __int_as_float(flags));
-            wb.qrng[nxt][rslot] = rng->s;
-        } else {
-            float4 l = wb.pathL[path];  // next-event radiance added so far
-            wb.pathL[path] = make_float4(l.x + L.x, l.y + L.y, l.z + L.z, __int_as_float(flags));
-        }
+    __device__ __forceinline__ void Done(bool c, const Ray& o, float lp, float ls, int f, V3 l) {
+        cont = c;
+        out = o;
+        lastPdf = lp;
+        lastSin = ls;
+        flags = f;
+        L = l;
     }
 };
 
@@ -780,29 +763,106 @@ __device__ __noinline__ float2 SettleTie(const DevJob& J, V3 o, V3 d, float2 h) 
     return make_float2(tb, __int_as_float(best));
 }
 
+__device__ __forceinline__ void CopyAsync16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void CopyAsync8(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void CopyAsyncWait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Bound by the latency of a chain of memory trips (660 instructions an entry, 31% of issue
+// slots busy at 15 warps per SM), so the chain is kept short: the next entry's state is on
+// its way into shared memory while this one is shaded, both appends of a warp go to the
+// counters in one instruction when all its lanes are done (two lanes, one counter each),
+// and a path that ends before any next-event ray could add to it writes its radiance
+// without reading it. Shade stage of the 1.0M-triangle 1080p frame: 13.78 ms with loads at
+// the start and two appends a step; one append 12.50, entries staged ahead 11.33, and at
+// 5 blocks of 102 registers instead of 4 10.21 ms (6 blocks 10.18, 7 11.29, 8 11.57).
 template <int kInteg>
-__global__ void __launch_bounds__(128, PT_SHADE_MIN_BLOCKS) ShadeKernel(const DevJob* __restrict__ jobs, WaveBuffers wb,
+__global__ void __launch_bounds__(128, kShadeBlocks) ShadeKernel(const DevJob* __restrict__ jobs, WaveBuffers wb,
                                                    int cur) {
+    __shared__ float4 sIn[4][kTraceBlock];  // the thread's next queue entry
+    __shared__ float2 sHit[kTraceBlock];
+    __shared__ unsigned long long sRng[kTraceBlock];
+    __shared__ float4 sShadow[4 * kTraceBlock];
     const int n = wb.counts[cur];
     const int nxt = cur ^ 1;
     const int sole = wb.desc->soleJob;
-    if (blockIdx.x == 0 && threadIdx.x == 0) wb.counts[4] = 0;  // the next extend fetches from zero
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 ra = wb.ray[cur][2 * i], rb = wb.ray[cur][2 * i + 1];
-        float2 h = wb.hit[i];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const unsigned below = (1u << lane) - 1u;
+    if (blockIdx.x == 0 && tid == 0) wb.counts[4] = 0;  // the next extend fetches from zero
+    auto stage = [&](int i) {
+        if (i < n) {
+            CopyAsync16(&sIn[0][tid], wb.ray[cur] + 2 * (size_t)i);
+            CopyAsync16(&sIn[1][tid], wb.ray[cur] + 2 * (size_t)i + 1);
+            CopyAsync16(&sIn[2][tid], wb.qs0[cur] + i);
+            CopyAsync16(&sIn[3][tid], wb.qs1[cur] + i);
+            CopyAsync8(&sHit[tid], wb.hit + i);
+            CopyAsync8(&sRng[tid], wb.qrng[cur] + i);
+        }
+    };
+    const int step = gridDim.x * kTraceBlock;
+    int i = blockIdx.x * kTraceBlock + tid;
+    stage(i);
+    for (; i - lane < n; i += step) {  // whole warps step together
+        CopyAsyncWait();
+        const float4 ra = sIn[0][tid], rb = sIn[1][tid], s0 = sIn[2][tid], s2 = sIn[3][tid];
+        float2 h = sHit[tid];
+        PathRng rng(sRng[tid]);
+        stage(i + step);  // the thread's own slots, read above
         const int path = __float_as_int(ra.w);
-        const DevJob& J = jobs[JobOf(wb.pathJob, sole, path)];
-        if (__float_as_int(h.y) < -1) h = SettleTie(J, V3(ra.x, ra.y, ra.z), V3(rb.x, rb.y, rb.z), h);
+        bool on = i < n;
+        StageSink sink;
+        sink.sh = sShadow + tid;
+        if (on) {
+            const DevJob& J = jobs[JobOf(wb.pathJob, sole, path)];
+            if (__float_as_int(h.y) < -1) h = SettleTie(J, V3(ra.x, ra.y, ra.z), V3(rb.x, rb.y, rb.z), h);
 #if PT_CHECK
-        if (__float_as_int(h.y) >= J.S.numTris || (unsigned)path >= (unsigned)wb.capacity) {
+            if (__float_as_int(h.y) >= J.S.numTris || (unsigned)path >= (unsigned)wb.capacity) {
+                atomicOr(wb.counts + 3, kErrBounds);
+                on = false;
+            }
+            if (on)
+#endif
+                ShadeOne<kInteg>(J, path, V3(ra.x, ra.y, ra.z), V3(rb.x, rb.y, rb.z), s0, s2, rb.w, h, rng, sink);
+        }
+        __syncwarp();
+        const unsigned rays = __ballot_sync(kFullMask, sink.cont), shadows = __ballot_sync(kFullMask, sink.shadow);
+        int base = 0;
+        if (lane < 2) {
+            const int add = __popc(lane ? shadows : rays);
+            if (add) base = atomicAdd(wb.counts + (lane ? 2 : nxt), add);
+        }
+        const int rslot = __shfl_sync(kFullMask, base, 0) + __popc(rays & below);
+        const int sslot = __shfl_sync(kFullMask, base, 1) + __popc(shadows & below);
+#if PT_CHECK
+        if ((sink.cont && rslot >= wb.capacity) || (sink.shadow && sslot >= wb.capacity)) {
             atomicOr(wb.counts + 3, kErrBounds);
-            continue;  // the appends are aggregated over the lanes that reach them
+            continue;
         }
 #endif
-        PathRng rng(wb.qrng[cur][i]);
-        StageSink sink{wb, nxt, path, &rng};
-        ShadeOne<kInteg>(J, path, V3(ra.x, ra.y, ra.z), V3(rb.x, rb.y, rb.z), wb.qs0[cur][i],
-                         wb.qs1[cur][i], rb.w, h, rng, sink);
+        if (sink.shadow) {
+            float4* e = wb.shadow + 4 * (size_t)sslot;
+            for (int k = 0; k < 4; k++) e[k] = sShadow[k * kTraceBlock + tid];
+        }
+        if (sink.cont) {
+            const Ray& out = sink.out;
+            wb.ray[nxt][2 * rslot] = make_float4(out.o.x, out.o.y, out.o.z, __int_as_float(path));
+            wb.ray[nxt][2 * rslot + 1] = make_float4(out.d.x, out.d.y, out.d.z, out.ior);
+            wb.qs0[nxt][rslot] = make_float4(out.T.x, out.T.y, out.T.z, out.prob);
+            wb.qs1[nxt][rslot] = make_float4(sink.lastPdf, sink.lastSin, __int_as_float(out.bounce),
+                                             __int_as_float(sink.flags));
+            wb.qrng[nxt][rslot] = rng.s;
+        } else if (on) {
+            // the radiance so far: next-event rays add it from the first bounce of a
+            // PathTracing path on, so a path that ends earlier only writes
+            float4 l = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (kInteg != kSimplePathTracing && __float_as_int(s2.z) > 0) l = wb.pathL[path];
+            wb.pathL[path] = make_float4(l.x + sink.L.x, l.y + sink.L.y, l.z + sink.L.z, __int_as_float(sink.flags));
+        }
     }
 }
 
@@ -1379,10 +1439,6 @@ int DefaultStageGrid() {
     return grid;
 }
 
-// Grid of the shade stage: PT_SHADE_BLOCKS_PER_SM blocks per SM (0: the trace grid).
-#ifndef PT_SHADE_BLOCKS_PER_SM
-#define PT_SHADE_BLOCKS_PER_SM 0
-#endif
 static int SmCount() {
     static int sms = 0;
     if (sms == 0) {
@@ -1392,12 +1448,12 @@ static int SmCount() {
     }
     return sms;
 }
-static int ShadeGrid(int traceGrid) {
-    return PT_SHADE_BLOCKS_PER_SM > 0 ? SmCount() * PT_SHADE_BLOCKS_PER_SM : traceGrid;
-}
-
 int StageGrid(const WaveTuning& tune) {
     return tune.blocksPerSm > 0 ? SmCount() * tune.blocksPerSm : DefaultStageGrid();
+}
+// Grid of the shade stage: its own resident blocks, or as many as asked for.
+static int ShadeGrid(const WaveTuning& tune) {
+    return SmCount() * (tune.blocksPerSm > 0 ? tune.blocksPerSm : kShadeBlocks);
 }
 
 // The bounce iterations [it0, it0 + count) of a wave (queue parity from it0).
@@ -1440,12 +1496,11 @@ static void LaunchTail(const DevJob* jobs, const WaveBuffers& wb, int integrator
 // wave may end in one earlier, where few paths are left.
 // envOnly: no job of the wave has area lights (the any-hit shadow kernel).
 static void LaunchBounces(const DevJob* jobs, const WaveUnit* units, const WaveBuffers& wb,
-                          int integrator, int grid, int it0, int count, cudaStream_t stream,
+                          int integrator, int grid, int sgrid, int it0, int count, cudaStream_t stream,
                           WaveProfile* prof, int* nl, bool sort, StageOverlap* ov, bool envOnly,
                           int tailFrom = -1, bool raster = false, bool mayTail = false) {
     StageEvents* ev = prof ? (StageEvents*)prof->events : nullptr;
     const int block = kTraceBlock;
-    const int sgrid = ShadeGrid(grid);
     bool pendingShadow = false;  // a shadow stage on the side stream the next shade must wait for
     for (int it = it0; it < it0 + count; it++) {
         // sorted bounces trace queue 0 and reorder the rays shade appends to queue 1 back into it
@@ -1634,7 +1689,7 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
                     const WaveTuning& tune, WaveGraphCache* graphs, int lane, bool accumulate) {
     if (shape.nPaths <= 0) return cudaSuccess;
     if (shape.nPaths > wb.capacity) return cudaErrorInvalidValue;
-    const int grid = StageGrid(tune);
+    const int grid = StageGrid(tune), sgrid = ShadeGrid(tune);
     const int block = kTraceBlock;
     StageEvents* ev = prof ? (StageEvents*)prof->events : nullptr;
     bool useGraphs = graphs && !prof && tune.graphs && stream != 0 && stream != cudaStreamLegacy;
@@ -1677,7 +1732,7 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
         const int iters = shape.iters >= 0 ? shape.iters : kMaxReplayBounces;
         auto record = [&](int* n) {
             RaygenKernel<<<grid, block, 0, stream>>>(jobs, units, wb, 0, raster ? 1 : 0);
-            LaunchBounces(jobs, units, wb, shape.integrator, grid, 0, iters, stream, prof, n, sort,
+            LaunchBounces(jobs, units, wb, shape.integrator, grid, sgrid, 0, iters, stream, prof, n, sort,
                           ov, envOnly, tailFrom, raster, !sort);
             if (accumulate) AccumulateKernel<<<grid, block, 0, stream>>>(jobs, units, wb);
             *n += accumulate ? 2 : 1;
@@ -1688,7 +1743,7 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
             if (ev) ev->Begin(0, stream);
             RaygenKernel<<<grid, block, 0, stream>>>(jobs, units, wb, 0, raster ? 1 : 0);
             if (ev) ev->End(0, stream);
-            LaunchBounces(jobs, units, wb, shape.integrator, grid, 0, iters, stream, prof, &nl, sort,
+            LaunchBounces(jobs, units, wb, shape.integrator, grid, sgrid, 0, iters, stream, prof, &nl, sort,
                           ov, envOnly, tailFrom, raster, !sort && !prof);
             if (accumulate) {
                 if (ev) ev->Begin(4, stream);
@@ -1719,12 +1774,12 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
                 WaveGraphKey k = key;
                 k.iters = -kPollEvery;
                 e = ReplayCaptured(graphs, k, stream, &nl, [&](int* n) {
-                    LaunchBounces(jobs, units, wb, shape.integrator, grid, 0, kPollEvery, stream, nullptr, n, sort,
+                    LaunchBounces(jobs, units, wb, shape.integrator, grid, sgrid, 0, kPollEvery, stream, nullptr, n, sort,
                                   ov, envOnly);
                 });
                 if (e != cudaSuccess) break;
             } else {
-                LaunchBounces(jobs, units, wb, shape.integrator, grid, it, kPollEvery, stream, prof, &nl, sort, ov,
+                LaunchBounces(jobs, units, wb, shape.integrator, grid, sgrid, it, kPollEvery, stream, prof, &nl, sort, ov,
                               envOnly);
             }
         }
