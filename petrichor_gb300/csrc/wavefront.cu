@@ -27,8 +27,8 @@
 namespace ptg {
 
 // Minimum resident blocks per SM requested from the register allocator for the
-// trace (extend/shadow) stages: 7 blocks of 72 registers; 8 of 64 (which spill), 6 and 5
-// measured 17.65, 17.30 and 17.85 ms against 16.90 for the closest hits of the
+// trace (extend/shadow) stages: 7 blocks of at most 72 registers; 8 of 64 (which spill), 6
+// and 5 measured 17.65, 17.30 and 17.85 ms against 16.90 for the closest hits of the
 // 1.0M-triangle 1080p frame.
 #ifndef PT_TRACE_MIN_BLOCKS
 #define PT_TRACE_MIN_BLOCKS 7
@@ -432,8 +432,14 @@ __device__ __forceinline__ int FindUnit(const WaveUnit* __restrict__ units, int 
 
 // raster != 0: the first bounce is rasterised (raster_primary.cuh), whose keys and tie
 // marks start empty here.
+// full: whole entries, for the tail kernel. Otherwise the first bounce is the shade stage's
+// (ShadeKernel<.., true>), which forms what is the same for every camera ray itself: the
+// weight's three components (one, kept in the ray's last word), its probability and index of
+// refraction, and the empty path state and radiance. Bound by HBM writes, then by issue: 56
+// bytes a path instead of 104 with its raster keys, 2.23 -> 1.69 ms for 132.7M paths, and
+// the first shade step 0.34 ms shorter.
 __global__ void RaygenKernel(const DevJob* __restrict__ jobs, const WaveUnit* __restrict__ units,
-                             WaveBuffers wb, int cur, int raster) {
+                             WaveBuffers wb, int cur, int raster, int full) {
     const WaveDesc wd = *wb.desc;
     const int n = wd.nPaths, nUnits = wd.nUnits;
     const RasterScratch rs = CarveRaster(wb, cur, 0);
@@ -457,11 +463,13 @@ __global__ void RaygenKernel(const DevJob* __restrict__ jobs, const WaveUnit* __
             rs.key2[i] = kNoKey;
         }
         wb.ray[cur][2 * i] = make_float4(ray.o.x, ray.o.y, ray.o.z, __int_as_float(i));
-        wb.ray[cur][2 * i + 1] = make_float4(ray.d.x, ray.d.y, ray.d.z, 1.0f);
-        wb.qs0[cur][i] = make_float4(ray.T.x, ray.T.y, ray.T.z, 1.0f);
-        wb.qs1[cur][i] = make_float4(0.f, 0.f, __int_as_float(0), __int_as_float(0));
+        wb.ray[cur][2 * i + 1] = make_float4(ray.d.x, ray.d.y, ray.d.z, full ? 1.0f : ray.T.x);
+        if (full) {
+            wb.qs0[cur][i] = make_float4(ray.T.x, ray.T.y, ray.T.z, 1.0f);
+            wb.qs1[cur][i] = make_float4(0.f, 0.f, __int_as_float(0), __int_as_float(0));
+            wb.pathL[i] = make_float4(0.f, 0.f, 0.f, __int_as_float(0));
+        }
         wb.qrng[cur][i] = rng.s;
-        wb.pathL[i] = make_float4(0.f, 0.f, 0.f, __int_as_float(0));
         if (wd.soleJob < 0) wb.pathJob[i] = u.job;  // read only where a wave mixes jobs (JobOf)
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -781,10 +789,12 @@ __device__ __forceinline__ void CopyAsyncWait() { asm volatile("cp.async.wait_al
 // without reading it. Shade stage of the 1.0M-triangle 1080p frame: 13.78 ms with loads at
 // the start and two appends a step; one append 12.50, entries staged ahead 11.33, and at
 // 5 blocks of 102 registers instead of 4 10.21 ms (6 blocks 10.18, 7 11.29, 8 11.57).
-template <int kInteg>
+// kFirst: the queue is raygen's, short entries (RaygenKernel); every path's radiance is
+// written here.
+template <int kInteg, bool kFirst>
 __global__ void __launch_bounds__(128, kShadeBlocks) ShadeKernel(const DevJob* __restrict__ jobs, WaveBuffers wb,
                                                    int cur) {
-    __shared__ float4 sIn[4][kTraceBlock];  // the thread's next queue entry
+    __shared__ float4 sIn[kFirst ? 2 : 4][kTraceBlock];  // the thread's next queue entry
     __shared__ float2 sHit[kTraceBlock];
     __shared__ unsigned long long sRng[kTraceBlock];
     __shared__ float4 sShadow[4 * kTraceBlock];
@@ -798,8 +808,10 @@ __global__ void __launch_bounds__(128, kShadeBlocks) ShadeKernel(const DevJob* _
         if (i < n) {
             CopyAsync16(&sIn[0][tid], wb.ray[cur] + 2 * (size_t)i);
             CopyAsync16(&sIn[1][tid], wb.ray[cur] + 2 * (size_t)i + 1);
-            CopyAsync16(&sIn[2][tid], wb.qs0[cur] + i);
-            CopyAsync16(&sIn[3][tid], wb.qs1[cur] + i);
+            if (!kFirst) {
+                CopyAsync16(&sIn[kFirst ? 0 : 2][tid], wb.qs0[cur] + i);
+                CopyAsync16(&sIn[kFirst ? 0 : 3][tid], wb.qs1[cur] + i);
+            }
             CopyAsync8(&sHit[tid], wb.hit + i);
             CopyAsync8(&sRng[tid], wb.qrng[cur] + i);
         }
@@ -809,7 +821,9 @@ __global__ void __launch_bounds__(128, kShadeBlocks) ShadeKernel(const DevJob* _
     stage(i);
     for (; i - lane < n; i += step) {  // whole warps step together
         CopyAsyncWait();
-        const float4 ra = sIn[0][tid], rb = sIn[1][tid], s0 = sIn[2][tid], s2 = sIn[3][tid];
+        const float4 ra = sIn[0][tid], rb = sIn[1][tid];
+        const float4 s0 = kFirst ? make_float4(rb.w, rb.w, rb.w, 1.0f) : sIn[kFirst ? 0 : 2][tid];
+        const float4 s2 = kFirst ? make_float4(0.f, 0.f, 0.f, 0.f) : sIn[kFirst ? 0 : 3][tid];
         float2 h = sHit[tid];
         PathRng rng(sRng[tid]);
         stage(i + step);  // the thread's own slots, read above
@@ -827,7 +841,8 @@ __global__ void __launch_bounds__(128, kShadeBlocks) ShadeKernel(const DevJob* _
             }
             if (on)
 #endif
-                ShadeOne<kInteg>(J, path, V3(ra.x, ra.y, ra.z), V3(rb.x, rb.y, rb.z), s0, s2, rb.w, h, rng, sink);
+                ShadeOne<kInteg>(J, path, V3(ra.x, ra.y, ra.z), V3(rb.x, rb.y, rb.z), s0, s2,
+                                   kFirst ? 1.0f : rb.w, h, rng, sink);
         }
         __syncwarp();
         const unsigned rays = __ballot_sync(kFullMask, sink.cont), shadows = __ballot_sync(kFullMask, sink.shadow);
@@ -856,14 +871,28 @@ __global__ void __launch_bounds__(128, kShadeBlocks) ShadeKernel(const DevJob* _
             wb.qs1[nxt][rslot] = make_float4(sink.lastPdf, sink.lastSin, __int_as_float(out.bounce),
                                              __int_as_float(sink.flags));
             wb.qrng[nxt][rslot] = rng.s;
-        } else if (on) {
-            // the radiance so far: next-event rays add it from the first bounce of a
-            // PathTracing path on, so a path that ends earlier only writes
+        }
+        if (on && (kFirst || !sink.cont)) {
+            // the radiance so far: next-event rays add to it from the first bounce of a
+            // PathTracing path on, so a path that ends at that bounce only writes (and one
+            // that goes on starts at zero)
             float4 l = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (kInteg != kSimplePathTracing && __float_as_int(s2.z) > 0) l = wb.pathL[path];
-            wb.pathL[path] = make_float4(l.x + sink.L.x, l.y + sink.L.y, l.z + sink.L.z, __int_as_float(sink.flags));
+            if (!kFirst && kInteg != kSimplePathTracing) l = wb.pathL[path];
+            if (!sink.cont) l = make_float4(l.x + sink.L.x, l.y + sink.L.y, l.z + sink.L.z, __int_as_float(sink.flags));
+            wb.pathL[path] = l;
         }
     }
+}
+
+template <bool kFirst>
+static void LaunchShade(const DevJob* jobs, const WaveBuffers& wb, int integrator, int cur, int grid,
+                        cudaStream_t stream) {
+    if (integrator == kPathTracing)
+        ShadeKernel<kPathTracing, kFirst><<<grid, kTraceBlock, 0, stream>>>(jobs, wb, cur);
+    else if (integrator == kSimplePathTracing)
+        ShadeKernel<kSimplePathTracing, kFirst><<<grid, kTraceBlock, 0, stream>>>(jobs, wb, cur);
+    else
+        ShadeKernel<-1, kFirst><<<grid, kTraceBlock, 0, stream>>>(jobs, wb, cur);
 }
 
 // A next-event entry's visibility ray (PathTracing.cpp:202-327): environment entries
@@ -1493,12 +1522,12 @@ static void LaunchTail(const DevJob* jobs, const WaveBuffers& wb, int integrator
 }
 
 // tailFrom >= 0: bounces from it0 + tailFrom on run in one TailKernel launch. mayTail: the
-// wave may end in one earlier, where few paths are left.
+// wave may end in one earlier, where few paths are left. first: the queue is raygen's.
 // envOnly: no job of the wave has area lights (the any-hit shadow kernel).
 static void LaunchBounces(const DevJob* jobs, const WaveUnit* units, const WaveBuffers& wb,
                           int integrator, int grid, int sgrid, int it0, int count, cudaStream_t stream,
                           WaveProfile* prof, int* nl, bool sort, StageOverlap* ov, bool envOnly,
-                          int tailFrom = -1, bool raster = false, bool mayTail = false) {
+                          bool first, int tailFrom = -1, bool raster = false, bool mayTail = false) {
     StageEvents* ev = prof ? (StageEvents*)prof->events : nullptr;
     const int block = kTraceBlock;
     bool pendingShadow = false;  // a shadow stage on the side stream the next shade must wait for
@@ -1546,12 +1575,8 @@ static void LaunchBounces(const DevJob* jobs, const WaveUnit* units, const WaveB
             cudaStreamWaitEvent(stream, ov->join, 0);
             pendingShadow = false;
         }
-        if (integrator == kPathTracing)
-            ShadeKernel<kPathTracing><<<sgrid, block, 0, stream>>>(jobs, wb, cur);
-        else if (integrator == kSimplePathTracing)
-            ShadeKernel<kSimplePathTracing><<<sgrid, block, 0, stream>>>(jobs, wb, cur);
-        else
-            ShadeKernel<-1><<<sgrid, block, 0, stream>>>(jobs, wb, cur);
+        if (first && at == 0) LaunchShade<true>(jobs, wb, integrator, cur, sgrid, stream);
+        else LaunchShade<false>(jobs, wb, integrator, cur, sgrid, stream);
         if (ev) {
             ev->End(2, stream);
             TallyKernel<<<1, 1, 0, stream>>>(wb.counts, cur, prof->devCounters);
@@ -1731,9 +1756,9 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
     if (shape.iters >= 0 || whole) {
         const int iters = shape.iters >= 0 ? shape.iters : kMaxReplayBounces;
         auto record = [&](int* n) {
-            RaygenKernel<<<grid, block, 0, stream>>>(jobs, units, wb, 0, raster ? 1 : 0);
+            RaygenKernel<<<grid, block, 0, stream>>>(jobs, units, wb, 0, raster ? 1 : 0, whole ? 1 : 0);
             LaunchBounces(jobs, units, wb, shape.integrator, grid, sgrid, 0, iters, stream, prof, n, sort,
-                          ov, envOnly, tailFrom, raster, !sort);
+                          ov, envOnly, true, tailFrom, raster, !sort);
             if (accumulate) AccumulateKernel<<<grid, block, 0, stream>>>(jobs, units, wb);
             *n += accumulate ? 2 : 1;
         };
@@ -1741,10 +1766,10 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
             e = ReplayCaptured(graphs, key, stream, &nl, record);
         } else {
             if (ev) ev->Begin(0, stream);
-            RaygenKernel<<<grid, block, 0, stream>>>(jobs, units, wb, 0, raster ? 1 : 0);
+            RaygenKernel<<<grid, block, 0, stream>>>(jobs, units, wb, 0, raster ? 1 : 0, whole ? 1 : 0);
             if (ev) ev->End(0, stream);
             LaunchBounces(jobs, units, wb, shape.integrator, grid, sgrid, 0, iters, stream, prof, &nl, sort,
-                          ov, envOnly, tailFrom, raster, !sort && !prof);
+                          ov, envOnly, true, tailFrom, raster, !sort && !prof);
             if (accumulate) {
                 if (ev) ev->Begin(4, stream);
                 AccumulateKernel<<<grid, block, 0, stream>>>(jobs, units, wb);
@@ -1756,7 +1781,7 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
     } else {
         // SimplePathTracing has no depth cap: run blocks of bounces until the queue drains
         if (ev) ev->Begin(0, stream);
-        RaygenKernel<<<grid, block, 0, stream>>>(jobs, units, wb, 0, 0);
+        RaygenKernel<<<grid, block, 0, stream>>>(jobs, units, wb, 0, 0, 0);
         if (ev) ev->End(0, stream);
         nl++;
         for (int it = 0;; it += kPollEvery) {
@@ -1772,15 +1797,15 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
             }
             if (useGraphs) {
                 WaveGraphKey k = key;
-                k.iters = -kPollEvery;
+                k.iters = -kPollEvery - (it == 0 ? 1 : 0);  // the first block shades raygen's entries
                 e = ReplayCaptured(graphs, k, stream, &nl, [&](int* n) {
                     LaunchBounces(jobs, units, wb, shape.integrator, grid, sgrid, 0, kPollEvery, stream, nullptr, n, sort,
-                                  ov, envOnly);
+                                  ov, envOnly, it == 0);
                 });
                 if (e != cudaSuccess) break;
             } else {
                 LaunchBounces(jobs, units, wb, shape.integrator, grid, sgrid, it, kPollEvery, stream, prof, &nl, sort, ov,
-                              envOnly);
+                              envOnly, it == 0);
             }
         }
         if (e == cudaSuccess && accumulate) {
@@ -1878,7 +1903,7 @@ cudaError_t RunPrimaryHits(const DevJob* jobs, const WaveUnit* units, const Wave
     cudaError_t e = cudaMemcpyAsync(wb.desc, &d, sizeof(d), cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(wb.counts, 0, 16 * sizeof(int), stream);
     if (e != cudaSuccess) return e;
-    RaygenKernel<<<grid, kTraceBlock, 0, stream>>>(jobs, units, wb, 0, raster ? 1 : 0);
+    RaygenKernel<<<grid, kTraceBlock, 0, stream>>>(jobs, units, wb, 0, raster ? 1 : 0, 0);
     ExtendKernel<<<grid, kTraceBlock, 0, stream>>>(jobs, wb, 0, raster ? 1 : 0);
     int nl = 3;
     if (raster) {
