@@ -75,6 +75,7 @@ struct LaneRay {
     float tmin, tmax, tBest;
     int best;  // slot of the closest hit; -1 none; -2 - slot when another hit tied it
     bool anyHit;
+    int tag;  // next-event rays: the entry's tag (path, area light)
     const float4* nodes;  // the lane's 4-wide tree (rays of different jobs share a warp)
     const float4* tris;
     int nearX, nearY, nearZ;  // byte offsets in a node of the planes the ray meets first
@@ -907,7 +908,8 @@ __device__ __forceinline__ void ShadowRay(const DevScene& S, float4 e0, float4 e
     r.o = V3(e0.x, e0.y, e0.z);
     r.d = V3(e1.x, e1.y, e1.z);
     r.tmin = 0.0f;
-    const bool env = __float_as_int(e1.w) >= 0;
+    r.tag = __float_as_int(e1.w);
+    const bool env = r.tag >= 0;
     r.anyHit = env;
     r.tmax = env ? kFltMax : e0.w + 0.05f;
 }
@@ -920,10 +922,8 @@ __device__ __noinline__ void ApplyAreaLight(const DevScene& S, const float4* e, 
 template <bool kEnvOnly = false>
 __device__ __forceinline__ void ApplyShadow(const DevScene& S, const float4* e, const LaneRay& r,
                                             float4* pathL) {
-    const float4 e1 = e[1];
-    const int tag = __float_as_int(e1.w);
-    const int path = tag & 0x7FFFFFFF;
-    if (kEnvOnly || tag >= 0) {  // environment: adds when unoccluded
+    const int path = r.tag & 0x7FFFFFFF;
+    if (kEnvOnly || r.tag >= 0) {  // environment: adds when unoccluded
         if (r.best != -1) return;
         const float4 e2 = e[2];
         float4 l = pathL[path];
@@ -981,7 +981,7 @@ struct ShadowQueue {
         ShadowRay(jobs[JobOf(pathJob, soleJob, __float_as_int(e1.w) & 0x7FFFFFFF)].S, e0, e1, r);
     }
     __device__ void Finish(int j, const LaneRay& r) const {
-        const int path = __float_as_int(entries[4 * j + 1].w) & 0x7FFFFFFF;
+        const int path = r.tag & 0x7FFFFFFF;
         ApplyShadow<kEnvOnly>(jobs[JobOf(pathJob, soleJob, path)].S, entries + 4 * j, r, pathL);
     }
 };
