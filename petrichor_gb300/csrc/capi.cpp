@@ -584,6 +584,8 @@ int pt_scene_upload(pt_context* ctx, const pt_scene_desc* d, pt_scene_id* out) {
         nodes[2 * i] = F4(n.lo[0], n.lo[1], n.lo[2], n.hi[0]);
         nodes[2 * i + 1] = F4(n.hi[1], n.hi[2], IntBits(a), IntBits(b));
     }
+    // the wide tree that follows starts on a 128-byte line, so each of its nodes is one
+    nodes.resize((nodes.size() + 7) / 8 * 8);
     // wide collapse for the throughput traversal
     std::vector<float> wideF;
     float wideEps = 0.0f;
