@@ -122,7 +122,8 @@ struct WaveShape {
     int areaLights = 1;  // 0: no job of the wave has area lights (next-event rays are any-hit)
     // > 0: the first bounce of units [rasterUnit0, nUnits) (paths [rasterFrom, nPaths)) may
     // be rasterised (raster_primary.cuh); raster = their per-triangle records in all
-    int raster = 0, rasterFrom = 0, rasterUnit0 = 0;
+    // and rasterSamples = their samples a pixel (mean)
+    int raster = 0, rasterFrom = 0, rasterUnit0 = 0, rasterSamples = 0;
 };
 // Launch configuration (all choices give the same films). 0 = default.
 struct WaveTuning {

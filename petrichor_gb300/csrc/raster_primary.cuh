@@ -11,7 +11,7 @@
 //          projected with the camera's own mapping, one pixel of margin for the sample
 //          offsets; the whole image when it reaches the camera plane); the rectangle is
 //          cut into row segments of at most kRasterSeg pixels, appended to a work list;
-//   visit  one warp per segment: the lanes step through the segment's (pixel, sample)
+//   visit  a group of lanes per segment, who step through the segment's (pixel, sample)
 //          pairs, test each direction against the cone, and for those inside run the
 //          exact triangle test of the traversal (TriIntersect) and keep the nearest hit
 //          with a 64-bit atomic minimum over {distance bits, slot};
@@ -30,7 +30,6 @@
 #pragma once
 
 constexpr int kRasterSeg = 32;   // pixels per work item (one row segment)
-constexpr int kRasterBatch = 2;  // (pixel, sample) pairs a lane loads before testing them
 constexpr int kRasterRecF4 = 4;    // float4 per per-triangle record
 constexpr unsigned long long kNoKey = ~0ull;
 constexpr unsigned kUncertain = 0x80000000u;  // key bit: the hit may lie outside its leaf box
@@ -261,6 +260,8 @@ __device__ __forceinline__ bool HitNearTriangle(const NearBox& b, V3 o, V3 d, fl
 // Visits one row segment of triangle k: every (pixel, sample) pair of the wave's unit.
 // Pixel (x, y) is pixel q = qrow + x * hb of the band order (PixelOfIndex), and its
 // samples are paths pathBase + q * sw + j, whose directions are in the ray queue.
+// kGroup lanes work on the segment, kBatch pairs a lane at a time.
+template <int kGroup, int kBatch>
 __device__ __forceinline__ void RasterSegment(const RasterScratch& rs, const float4* __restrict__ rays,
                                              const DevScene& S, int k, int rec, int y,
                                              int xa, int xb, int W, int H, int band, int pathBase,
@@ -273,18 +274,18 @@ __device__ __forceinline__ void RasterSegment(const RasterScratch& rs, const flo
     const int y0 = (y / band) * band, hb = min(band, H - y0);
     const size_t qrow = (size_t)y0 * W + (y - y0);
     const int n = (xb - xa + 1) * sw;
-    // (pixel, sample) of pair f = lane + 32 i, advanced without a division per pair
-    const int dq = 32 / sw, dr = 32 % sw;
+    // (pixel, sample) of pair f = lane + kGroup i, advanced without a division per pair
+    const int dq = kGroup / sw, dr = kGroup % sw;
     int x = xa + lane / sw, j = lane % sw;
-    // kRasterBatch pairs per lane at a time: their directions are loaded before any is
+    // kBatch pairs per lane at a time: their directions are loaded before any is
     // tested, so the loads' latencies overlap; the minima are fire-and-forget reductions
-    for (int f0 = lane; f0 < n; f0 += 32 * kRasterBatch) {
-        float4 dv[kRasterBatch];
-        size_t idx[kRasterBatch];
+    for (int f0 = lane; f0 < n; f0 += kGroup * kBatch) {
+        float4 dv[kBatch];
+        size_t idx[kBatch];
 #pragma unroll
-        for (int b = 0; b < kRasterBatch; b++) {
+        for (int b = 0; b < kBatch; b++) {
             idx[b] = (size_t)pathBase + (qrow + (size_t)x * hb) * sw + j;
-            if (f0 + 32 * b < n) dv[b] = __ldg(rays + 2 * idx[b] + 1);
+            if (f0 + kGroup * b < n) dv[b] = __ldg(rays + 2 * idx[b] + 1);
             j += dr;
             x += dq;
             if (j >= sw) {
@@ -293,8 +294,8 @@ __device__ __forceinline__ void RasterSegment(const RasterScratch& rs, const flo
             }
         }
 #pragma unroll
-        for (int b = 0; b < kRasterBatch; b++) {
-            if (f0 + 32 * b >= n) break;
+        for (int b = 0; b < kBatch; b++) {
+            if (f0 + kGroup * b >= n) break;
             const float c0 = r0.x * dv[b].x + r0.y * dv[b].y + r0.z * dv[b].z + r0.w;
             const float c1 = r1.x * dv[b].x + r1.y * dv[b].y + r1.z * dv[b].z + r1.w;
             const float c2 = r2.x * dv[b].x + r2.y * dv[b].y + r2.z * dv[b].z + r2.w;
@@ -316,24 +317,37 @@ __device__ __forceinline__ void RasterSegment(const RasterScratch& rs, const flo
 }
 
 // One work item's (row segment's) unit: its job's scene, camera and image, its paths.
+template <int kGroup, int kBatch>
 __device__ __forceinline__ void RasterItem(const DevJob* __restrict__ jobs, const WaveUnit& u,
                                           const RasterScratch& rs, const float4* __restrict__ rays,
                                           int band, int k, int y, int xa, int xb, int lane) {
     const DevJob& J = jobs[u.job];
     const float tmin = J.st.integrator == kSimplePathTracing ? kEps : 0.0f;
-    RasterSegment(rs, rays, J.S, k, u.recBase + k, y, xa, xb, J.st.width, J.st.height, band,
+    RasterSegment<kGroup, kBatch>(rs, rays, J.S, k, u.recBase + k, y, xa, xb, J.st.width, J.st.height, band,
                   u.pathBase, u.sw, LoadV3(J.C.pos), tmin, lane);
 }
 
-__global__ void __launch_bounds__(128) RasterVisitKernel(const DevJob* __restrict__ jobs,
+// Bound by memory latency and, with few samples a pixel, by idle lanes: a triangle covers a
+// few pixels of a row, so its (pixel, sample) pairs fill a warp only where a pixel has many
+// samples. kGroup lanes take an item. Raster stage (1920x1080) with 32 lanes and 2 pairs a
+// lane; 8 lanes, 2 pairs, 8 blocks per SM; 32 lanes, 1 pair, 8 blocks:
+//    1 sample  a pixel,    30,000 triangles  0.207  0.102  0.172 ms
+//    4                    100,000            0.497  0.272  0.386
+//    8                    500,000            1.47   0.76   1.09
+//   16                       1.0M            2.66   1.79   2.12
+//   32                       1.0M            3.43   3.62   2.91
+//   64                       1.0M            5.27   6.83   5.38
+// (RasterVisit picks by the wave's samples a pixel.)
+template <int kGroup, int kBatch, int kMinBlocks>
+__global__ void __launch_bounds__(128, kMinBlocks) RasterVisitKernel(const DevJob* __restrict__ jobs,
                                                          const WaveUnit* __restrict__ units,
                                                          WaveBuffers wb, int cur) {
     const WaveDesc wd = *wb.desc;
     const RasterScratch rs = CarveRaster(wb, cur, wd.rasterRecs);
     const float4* rays = wb.ray[cur];
-    const int lane = threadIdx.x & 31;
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
+    const int lane = threadIdx.x & (kGroup - 1);
+    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / kGroup;
+    const long long warps = ((long long)gridDim.x * blockDim.x) / kGroup;
     long long nItems = *reinterpret_cast<const long long*>(wb.counts + 8);
     if (nItems > rs.itemCap) nItems = rs.itemCap;
     // the next item is loaded while the current one is visited
@@ -347,7 +361,7 @@ __global__ void __launch_bounds__(128) RasterVisitKernel(const DevJob* __restric
 #if PT_CHECK
         if (k < 0 || k >= jobs[u.job].S.numTris) continue;
 #endif
-        RasterItem(jobs, u, rs, rays, wd.band, k, y, (int)(it.w & 0xffffu), (int)(it.w >> 16), lane);
+        RasterItem<kGroup, kBatch>(jobs, u, rs, rays, wd.band, k, y, (int)(it.w & 0xffffu), (int)(it.w >> 16), lane);
     }
     // triangles whose items did not fit in the list: whole, one warp each
     const int nOver = wb.counts[10];
@@ -359,7 +373,7 @@ __global__ void __launch_bounds__(128) RasterVisitKernel(const DevJob* __restric
                   y1 = __float_as_int(r3.w);
         for (int y = y0; y <= y1; y++)
             for (int xa = x0; xa <= x1; xa += kRasterSeg)
-                RasterItem(jobs, u, rs, rays, wd.band, ov.x, y, xa, min(x1, xa + kRasterSeg - 1), lane);
+                RasterItem<kGroup, kBatch>(jobs, u, rs, rays, wd.band, ov.x, y, xa, min(x1, xa + kRasterSeg - 1), lane);
     }
 }
 

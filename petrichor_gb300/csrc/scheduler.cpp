@@ -121,6 +121,8 @@ void PrepareRasterUnits(const std::vector<DevJob>& jobs, std::vector<WaveUnit>* 
         pixels += P;
     }
     shape->rasterUnit0 = (int)trace.size();
+    const int firstPixel = (*units)[trace.size()].pixelBase;
+    shape->rasterSamples = (paths - shape->rasterFrom) / std::max(1, pixels - firstPixel);
 }
 
 std::vector<ServePick> PlanServeWave(const std::vector<ServeRequestView>& reqs,

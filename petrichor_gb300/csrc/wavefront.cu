@@ -1510,6 +1510,19 @@ struct StageOverlap {
     }
 };
 
+// The visit kernel's form by the rasterised units' samples a pixel (figures at the kernel):
+// 0 up to 16, 1 up to 63, 2 from 64 on.
+static int RasterVisitClass(const WaveShape& shape) {
+    return shape.rasterSamples <= 16 ? 0 : shape.rasterSamples < 64 ? 1 : 2;
+}
+static void RasterVisit(const DevJob* jobs, const WaveUnit* units, const WaveBuffers& wb, int cur, int visit,
+                        cudaStream_t stream) {
+    const int grid = SmCount() * 16;
+    if (visit == 0) RasterVisitKernel<8, 2, 8><<<grid, kTraceBlock, 0, stream>>>(jobs, units, wb, cur);
+    else if (visit == 1) RasterVisitKernel<32, 1, 8><<<grid, kTraceBlock, 0, stream>>>(jobs, units, wb, cur);
+    else RasterVisitKernel<32, 2, 1><<<grid, kTraceBlock, 0, stream>>>(jobs, units, wb, cur);
+}
+
 static void LaunchTail(const DevJob* jobs, const WaveBuffers& wb, int integrator, int cur, int iters,
                        int most, cudaStream_t stream) {
     const int grid = SmCount() * kTailBlocksPerSm;
@@ -1523,11 +1536,13 @@ static void LaunchTail(const DevJob* jobs, const WaveBuffers& wb, int integrator
 
 // tailFrom >= 0: bounces from it0 + tailFrom on run in one TailKernel launch. mayTail: the
 // wave may end in one earlier, where few paths are left. first: the queue is raygen's.
+// visit: the raster visit kernel's form.
 // envOnly: no job of the wave has area lights (the any-hit shadow kernel).
 static void LaunchBounces(const DevJob* jobs, const WaveUnit* units, const WaveBuffers& wb,
                           int integrator, int grid, int sgrid, int it0, int count, cudaStream_t stream,
                           WaveProfile* prof, int* nl, bool sort, StageOverlap* ov, bool envOnly,
-                          bool first, int tailFrom = -1, bool raster = false, bool mayTail = false) {
+                          bool first, int tailFrom = -1, bool raster = false, bool mayTail = false,
+                          int visit = 0) {
     StageEvents* ev = prof ? (StageEvents*)prof->events : nullptr;
     const int block = kTraceBlock;
     bool pendingShadow = false;  // a shadow stage on the side stream the next shade must wait for
@@ -1553,7 +1568,7 @@ static void LaunchBounces(const DevJob* jobs, const WaveUnit* units, const WaveB
                 ev->Begin(5, stream);
             }
             RasterSetupKernel<<<SmCount() * 32, block, 0, stream>>>(jobs, units, wb, cur);
-            RasterVisitKernel<<<SmCount() * 16, block, 0, stream>>>(jobs, units, wb, cur);
+            RasterVisit(jobs, units, wb, cur, visit, stream);
             RasterFinishKernel<<<grid, block, 0, stream>>>(wb, cur);
             // few paths, if any: a small grid (an empty launch of the full one took 0.12 ms)
             RetraceKernel<<<2 * SmCount(), block, 0, stream>>>(jobs, wb, cur);
@@ -1751,14 +1766,15 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
     StageOverlap* ov =
       (graphs && !prof && graphs->overlap[lane & 1].Ready()) ? &graphs->overlap[lane & 1] : nullptr;
     const bool envOnly = !shape.areaLights;
+    const int visit = RasterVisitClass(shape);
     const WaveGraphKey key{jobs, units, wb.ray[0], wb.capacity, shape.iters, shape.integrator, grid,
-                           sort ? 1 : 0, accumulate ? 1 : 0, tailFrom, raster ? 1 : 0, envOnly ? 1 : 0};
+                           sort ? 1 : 0, accumulate ? 1 : 0, tailFrom, raster ? 1 + visit : 0, envOnly ? 1 : 0};
     if (shape.iters >= 0 || whole) {
         const int iters = shape.iters >= 0 ? shape.iters : kMaxReplayBounces;
         auto record = [&](int* n) {
             RaygenKernel<<<grid, block, 0, stream>>>(jobs, units, wb, 0, raster ? 1 : 0, whole ? 1 : 0);
             LaunchBounces(jobs, units, wb, shape.integrator, grid, sgrid, 0, iters, stream, prof, n, sort,
-                          ov, envOnly, true, tailFrom, raster, !sort);
+                          ov, envOnly, true, tailFrom, raster, !sort, visit);
             if (accumulate) AccumulateKernel<<<grid, block, 0, stream>>>(jobs, units, wb);
             *n += accumulate ? 2 : 1;
         };
@@ -1769,7 +1785,7 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
             RaygenKernel<<<grid, block, 0, stream>>>(jobs, units, wb, 0, raster ? 1 : 0, whole ? 1 : 0);
             if (ev) ev->End(0, stream);
             LaunchBounces(jobs, units, wb, shape.integrator, grid, sgrid, 0, iters, stream, prof, &nl, sort,
-                          ov, envOnly, true, tailFrom, raster, !sort && !prof);
+                          ov, envOnly, true, tailFrom, raster, !sort && !prof, visit);
             if (accumulate) {
                 if (ev) ev->Begin(4, stream);
                 AccumulateKernel<<<grid, block, 0, stream>>>(jobs, units, wb);
@@ -1908,7 +1924,7 @@ cudaError_t RunPrimaryHits(const DevJob* jobs, const WaveUnit* units, const Wave
     int nl = 3;
     if (raster) {
         RasterSetupKernel<<<SmCount() * 32, kTraceBlock, 0, stream>>>(jobs, units, wb, 0);
-        RasterVisitKernel<<<SmCount() * 16, kTraceBlock, 0, stream>>>(jobs, units, wb, 0);
+        RasterVisit(jobs, units, wb, 0, RasterVisitClass(shape), stream);
         RasterFinishKernel<<<grid, kTraceBlock, 0, stream>>>(wb, 0);
         RetraceKernel<<<2 * SmCount(), kTraceBlock, 0, stream>>>(jobs, wb, 0);
         nl += 4;
