@@ -13,11 +13,22 @@ struct DeviceBuildStats {
     int levels = 0, rounds = 0, heapsorts = 0, launches = 0;
 };
 
+// A build's device arrays, kept for the caller: all in one allocation, to be freed with
+// cudaFree(block).
+struct DeviceBvh {
+    void* block = nullptr;
+    const float* positions = nullptr;
+    const int32_t* indices = nullptr;
+    const BvhNodeOut* nodes = nullptr;
+    const int32_t* primIds = nullptr;
+};
+
 // positions: numVertices x 3 floats, indices: numTriangles x 3 (host memory, validated
 // by the caller). Allocates its scratch (about 250 bytes per triangle) for the build
-// and frees it; synchronises `stream`. On failure `out` is empty and `error` says why.
+// in one piece and frees it, or hands it to `keep` (null: not kept; left alone when there are
+// no triangles); synchronises `stream`. On failure `out` is empty and `error` says why.
 cudaError_t BuildBinnedSahDevice(const float* positions, int numVertices, const int32_t* indices,
                                  int numTriangles, cudaStream_t stream, BvhResult* out,
-                                 std::string* error, DeviceBuildStats* stats);
+                                 std::string* error, DeviceBuildStats* stats, DeviceBvh* keep = nullptr);
 
 }  // namespace ptg

@@ -17,7 +17,6 @@
 #include <memory>
 #include <mutex>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "bvh_builder.h"
@@ -26,6 +25,7 @@
 #include "pt_kernels.h"
 #include "pt_layout.h"
 #include "context.h"
+#include "scene_records.h"
 #include "scheduler.h"
 
 using namespace ptg;
@@ -43,26 +43,6 @@ int CudaFail(pt_context* ctx, cudaError_t e, const char* what) {
                         e == cudaErrorHardwareStackError;
     return Fail(ctx, sticky ? PT_ERR_DEVICE_FAULT : PT_ERR_CUDA,
                 std::string(what) + ": " + cudaGetErrorString(e));
-}
-
-// fn(i) for i in [0, n) on the host's cores (serially for small n); fn must be safe to
-// run concurrently for different i.
-template <class F>
-void ParallelFor(size_t n, F&& fn) {
-    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
-    const size_t nt = std::min<size_t>(hw, n / 65536 + 1);
-    if (nt <= 1) {
-        for (size_t i = 0; i < n; i++) fn(i);
-        return;
-    }
-    std::vector<std::thread> pool;
-    const size_t chunk = (n + nt - 1) / nt;
-    for (size_t t = 0; t < nt; t++)
-        pool.emplace_back([&, t] {
-            const size_t e = std::min(n, (t + 1) * chunk);
-            for (size_t i = t * chunk; i < e; i++) fn(i);
-        });
-    for (std::thread& th : pool) th.join();
 }
 
 int Alloc(pt_context* ctx, DeviceBuffer& b, size_t bytes) {
@@ -96,19 +76,28 @@ void Free(pt_context* ctx, DeviceBuffer& b) {
     b.bytes = 0;
 }
 
+// A scene's buffer of `bytes`, kept with the scene.
 template <typename T>
-int Upload(pt_context* ctx, SceneGpu& s, const std::vector<T>& host, const T** devOut) {
+int SceneBuffer(pt_context* ctx, SceneGpu& s, size_t bytes, T** devOut) {
     DeviceBuffer b;
-    const size_t bytes = std::max<size_t>(host.size() * sizeof(T), 16);
-    int rc = Alloc(ctx, b, bytes);
+    const int rc = Alloc(ctx, b, std::max<size_t>(bytes, 16));
     if (rc != PT_OK) return rc;
     s.buffers.push_back(b);
+    *devOut = (T*)b.ptr;
+    return PT_OK;
+}
+
+template <typename T>
+int Upload(pt_context* ctx, SceneGpu& s, const std::vector<T>& host, const T** devOut) {
+    T* p = nullptr;
+    const int rc = SceneBuffer(ctx, s, host.size() * sizeof(T), &p);
+    if (rc != PT_OK) return rc;
     if (!host.empty()) {
         const cudaError_t e =
-          cudaMemcpyAsync(b.ptr, host.data(), host.size() * sizeof(T), cudaMemcpyHostToDevice, ctx->stream);
+          cudaMemcpyAsync(p, host.data(), host.size() * sizeof(T), cudaMemcpyHostToDevice, ctx->stream);
         if (e != cudaSuccess) return CudaFail(ctx, e, "scene upload");
     }
-    *devOut = (const T*)b.ptr;
+    *devOut = p;
     return PT_OK;
 }
 
@@ -564,10 +553,19 @@ int pt_scene_upload(pt_context* ctx, const pt_scene_desc* d, pt_scene_id* out) {
     const int T = (int)d->num_triangles;
     const auto t0 = std::chrono::steady_clock::now();
     BvhResult bvh;
+    DeviceBvh kept;  // the build's device arrays, from which the scene's records are formed
+    // device memory of this call alone; freed after the stream has run (cudaFree waits)
+    struct Temporary {
+        std::vector<void*> ptrs;
+        ~Temporary() {
+            for (void* p : ptrs) cudaFree(p);
+        }
+    } temporary;
     if (ctx->bvhBuilder == PT_BVH_BUILDER_DEVICE) {
         std::string why;
         const cudaError_t be = BuildBinnedSahDevice(d->positions, (int)d->num_vertices, d->indices, T,
-                                                    ctx->stream, &bvh, &why, nullptr);
+                                                    ctx->stream, &bvh, &why, nullptr, &kept);
+        temporary.ptrs.push_back(kept.block);
         if (be != cudaSuccess)
             return Fail(ctx, be == cudaErrorMemoryAllocation ? PT_ERR_OUT_OF_MEMORY : PT_ERR_CUDA, why);
     } else {
@@ -575,96 +573,27 @@ int pt_scene_upload(pt_context* ctx, const pt_scene_desc* d, pt_scene_id* out) {
     }
     const double buildSec =
       std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-    // nodes
-    std::vector<float4> nodes(bvh.nodes.size() * 2);
-    for (size_t i = 0; i < bvh.nodes.size(); i++) {
-        const BvhNodeOut& n = bvh.nodes[i];
-        const int32_t a = n.leaf ? n.begin : n.child[0];
-        const int32_t b = n.leaf ? (n.end - n.begin) : -1;
-        nodes[2 * i] = F4(n.lo[0], n.lo[1], n.lo[2], n.hi[0]);
-        nodes[2 * i + 1] = F4(n.hi[1], n.hi[2], IntBits(a), IntBits(b));
-    }
-    // the wide tree that follows starts on a 128-byte line, so each of its nodes is one
-    nodes.resize((nodes.size() + 7) / 8 * 8);
     // wide collapse for the throughput traversal
     std::vector<float> wideF;
     float wideEps = 0.0f;
     if (!CollapseWide(bvh, &wideF, kWide, &wideEps))
         return Fail(ctx, PT_ERR_UNSUPPORTED, "too many triangles for the wide BVH leaf encoding");
-    std::vector<float4> wide(wideF.size() / 4);
-    std::memcpy(wide.data(), wideF.data(), wideF.size() * sizeof(float));
-    // the binary leaf node of every primitive slot, as an offset in float4 from the wide
-    // tree (stored after the binary nodes): its widened box bounds where the throughput
-    // traversal counts a hit (a hit before the ray enters that box is not one)
-    std::vector<int32_t> boxOf((size_t)T, 0);
-    for (size_t i = 0; i < bvh.nodes.size(); i++)
-        if (bvh.nodes[i].leaf)
-            for (int k = bvh.nodes[i].begin; k < bvh.nodes[i].end; k++)
-                boxOf[(size_t)k] = (int32_t)(2 * i) - (int32_t)nodes.size();
-    // triangles in leaf order
-    std::vector<float4> tris((size_t)T * 3);
-    ParallelFor((size_t)T, [&](size_t kk) {
-        const int k = (int)kk;
-        const int t = bvh.primIds[k];
-        const HV3 v0 = Load(d->positions + 3 * d->indices[3 * t]);
-        const HV3 e1 = Sub(Load(d->positions + 3 * d->indices[3 * t + 1]), v0);
-        const HV3 e2 = Sub(Load(d->positions + 3 * d->indices[3 * t + 2]), v0);
-        tris[3 * (size_t)k] = F4(v0.x, v0.y, v0.z, e1.x);
-        tris[3 * (size_t)k + 1] = F4(e1.y, e1.z, e2.x, e2.y);
-        tris[3 * (size_t)k + 2] = F4(e2.z, IntBits(t), IntBits(boxOf[(size_t)k]), wideEps);
-    });
-    // shading records, also in leaf order: a hit's slot addresses both records
-    // without a dependent read of the triangle id
-    std::vector<float4> shade((size_t)T * 3);
-    ParallelFor((size_t)T, [&](size_t kk) {
-        const int k = (int)kk;
-        const int t = bvh.primIds[k];
-        HV3 n[3] = {{0, 0, 1}, {0, 0, 1}, {0, 0, 1}};
-        if (d->normals)
-            for (int v = 0; v < 3; v++) n[v] = Load(d->normals + 3 * d->indices[3 * t + v]);
-        const int smooth = d->tri_shading ? (d->tri_shading[t] ? 1 : 0) : 0;
-        shade[3 * (size_t)k] = F4(n[0].x, n[0].y, n[0].z, IntBits(d->tri_material[t]));
-        shade[3 * (size_t)k + 1] = F4(n[1].x, n[1].y, n[1].z, IntBits(smooth));
-        shade[3 * (size_t)k + 2] = F4(n[2].x, n[2].y, n[2].z, 0.0f);
-    });
     // vertex uvs in leaf order, for the UV pass and texture maps (omitted when the
     // scene has neither)
     bool anyTex = false;
     for (uint32_t m = 0; m < d->num_materials; m++) anyTex = anyTex || HasTextureMaps(d->materials[m]);
-    std::vector<float4> uvs;
     bool anyUV = false;
     if (d->uvs)
         for (size_t i = 0; i < (size_t)d->num_vertices * 3 && !anyUV; i++) anyUV = d->uvs[i] != 0.0f;
-    if (anyUV || anyTex) {
-        uvs.assign((size_t)std::max(T, 1) * 3, F4(0.0f, 0.0f, 0.0f, 0.0f));
-        if (d->uvs)
-            ParallelFor((size_t)T, [&](size_t k) {
-                const int t = bvh.primIds[k];
-                for (int v = 0; v < 3; v++) {
-                    const float* u = d->uvs + 3 * (size_t)d->indices[3 * t + v];
-                    uvs[3 * k + v] = F4(u[0], u[1], u[2], 0.0f);
-                }
-            });
-    }
     // material texture maps: texels as {r, g, b, 0}, one texture after another
-    std::vector<float4> texels(1, F4(0.0f, 0.0f, 0.0f, 0.0f));
+    size_t numTexels = 0;
     std::vector<int4> texInfo(std::max<uint32_t>(d->num_textures, 1), int4{0, 0, 0, 0});
-    if (anyTex) {
-        size_t total = 0;
+    if (anyTex)
         for (uint32_t t = 0; t < d->num_textures; t++) {
             const pt_texture& X = d->textures[t];
-            texInfo[t] = int4{(int)total, X.width, X.height, 0};
-            total += (size_t)X.width * X.height;
+            texInfo[t] = int4{(int)numTexels, X.width, X.height, 0};
+            numTexels += (size_t)X.width * X.height;
         }
-        texels.assign(std::max<size_t>(total, 1), F4(0.0f, 0.0f, 0.0f, 0.0f));
-        for (uint32_t t = 0; t < d->num_textures; t++) {
-            const pt_texture& X = d->textures[t];
-            float4* dst = texels.data() + texInfo[t].x;
-            ParallelFor((size_t)X.width * X.height, [&](size_t i) {
-                dst[i] = F4(X.rgb[3 * i], X.rgb[3 * i + 1], X.rgb[3 * i + 2], 0.0f);
-            });
-        }
-    }
     // materials
     std::vector<DevMaterial> mats(d->num_materials);
     for (uint32_t m = 0; m < d->num_materials; m++) {
@@ -703,36 +632,82 @@ int pt_scene_upload(pt_context* ctx, const pt_scene_desc* d, pt_scene_id* out) {
         const float pdfAreaEach = 1.0f / (0.5f * Length(Cross(e0, e1)));
         sumArea += 1.0f / pdfAreaEach;
     }
+    // binary nodes and wide tree in one allocation, the wide tree right after the nodes and
+    // on a 128-byte line, so each of its nodes is one
+    const size_t wideOffset = (bvh.nodes.size() * 2 + 7) / 8 * 8;
     // environment texels (the importance-sampling row tables of
     // Environment::PreCalcCumulativeDistTex depend on H alone; the kernels evaluate them)
     const int W = d->env_width, H = d->env_height;
-    std::vector<float4> env((size_t)std::max(W * H, 1));
-    if (W > 0)
-        ParallelFor((size_t)W * H, [&](size_t i) {
-            env[i] = F4(d->env_rgb[3 * i], d->env_rgb[3 * i + 1], d->env_rgb[3 * i + 2], 0.0f);
-        });
     SceneGpu& s = *sg;
     DevScene& D = s.dev;
-    // binary nodes and wide tree in one allocation, the wide tree right after the nodes
-    std::vector<float4> tree;
-    tree.reserve(nodes.size() + wide.size());
-    tree.insert(tree.end(), nodes.begin(), nodes.end());
-    tree.insert(tree.end(), wide.begin(), wide.end());
-    if ((rc = Upload(ctx, s, tree, &D.nodes)) != PT_OK ||
-        (rc = Upload(ctx, s, tris, &D.tris)) != PT_OK ||
-        (rc = Upload(ctx, s, shade, &D.shade)) != PT_OK ||
-        (rc = Upload(ctx, s, mats, &D.mats)) != PT_OK ||
-        (rc = Upload(ctx, s, lights, &D.lights)) != PT_OK ||
-        (rc = Upload(ctx, s, env, &D.env)) != PT_OK ||
-        (anyTex && (rc = Upload(ctx, s, texels, &D.texels)) != PT_OK) ||
+    float4 *tree = nullptr, *tris = nullptr, *shade = nullptr, *env = nullptr, *texels = nullptr, *uvs = nullptr;
+    const size_t slot3 = 3 * sizeof(float4);
+    const bool withUV = anyUV || anyTex;
+    if ((rc = SceneBuffer(ctx, s, wideOffset * sizeof(float4) + wideF.size() * sizeof(float), &tree)) != PT_OK ||
+        (rc = SceneBuffer(ctx, s, (size_t)T * slot3, &tris)) != PT_OK ||
+        (rc = SceneBuffer(ctx, s, (size_t)T * slot3, &shade)) != PT_OK ||
+        (rc = Upload(ctx, s, mats, &D.mats)) != PT_OK || (rc = Upload(ctx, s, lights, &D.lights)) != PT_OK ||
+        (rc = SceneBuffer(ctx, s, std::max<size_t>((size_t)W * H, 1) * sizeof(float4), &env)) != PT_OK ||
+        (anyTex && (rc = SceneBuffer(ctx, s, std::max<size_t>(numTexels, 1) * sizeof(float4), &texels)) != PT_OK) ||
         (anyTex && (rc = Upload(ctx, s, texInfo, &D.texInfo)) != PT_OK) ||
-        ((anyUV || anyTex) && (rc = Upload(ctx, s, uvs, &D.uvs)) != PT_OK)) {
+        (withUV && (rc = SceneBuffer(ctx, s, (size_t)std::max(T, 1) * slot3, &uvs)) != PT_OK)) {
         for (auto& b : s.buffers) Free(ctx, b);
         return rc;
     }
-    D.wide = D.nodes + nodes.size();
+    D.nodes = tree;
+    D.tris = tris;
+    D.shade = shade;
+    D.env = env;
+    D.texels = texels;
+    D.uvs = uvs;
+    // the caller's arrays on the device, for the kernels that form the records
+    cudaError_t e = cudaSuccess;
+    auto lift = [&](const void* host, size_t bytes) -> void* {
+        void* p = nullptr;
+        if (!host || bytes == 0 || e != cudaSuccess) return nullptr;
+        e = cudaMalloc(&p, bytes);
+        if (e != cudaSuccess) return nullptr;
+        temporary.ptrs.push_back(p);
+        e = cudaMemcpyAsync(p, host, bytes, cudaMemcpyHostToDevice, ctx->stream);
+        return p;
+    };
+    const size_t V3 = 3 * sizeof(float) * (size_t)d->num_vertices, T1 = (size_t)T;
+    SceneArrays in{};
+    in.positions = kept.block ? kept.positions : (const float*)lift(d->positions, V3);
+    in.indices = kept.block ? kept.indices : (const int32_t*)lift(d->indices, 3 * sizeof(int32_t) * T1);
+    in.nodes = kept.block ? kept.nodes : (const BvhNodeOut*)lift(bvh.nodes.data(), bvh.nodes.size() * sizeof(BvhNodeOut));
+    in.primIds = kept.block ? kept.primIds : (const int32_t*)lift(bvh.primIds.data(), sizeof(int32_t) * T1);
+    in.normals = (const float*)lift(T > 0 ? d->normals : nullptr, V3);
+    in.uvs = (const float*)lift(T > 0 && withUV ? d->uvs : nullptr, V3);
+    in.material = (const int32_t*)lift(d->tri_material, sizeof(int32_t) * T1);
+    in.shading = (const uint8_t*)lift(d->tri_shading, T1);
+    in.numNodes = (int)bvh.nodes.size();
+    in.numTris = T;
+    if (e == cudaSuccess && !wideF.empty())
+        e = cudaMemcpyAsync(tree + wideOffset, wideF.data(), wideF.size() * sizeof(float), cudaMemcpyHostToDevice,
+                            ctx->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(env, 0, sizeof(float4), ctx->stream);
+    if (e == cudaSuccess && uvs) e = cudaMemsetAsync(uvs, 0, slot3, ctx->stream);
+    if (e == cudaSuccess) e = FormSceneRecords(in, tree, (int)wideOffset, wideEps, tris, shade, uvs, ctx->stream);
+    if (e == cudaSuccess && W > 0) {
+        const float* rgb = (const float*)lift(d->env_rgb, 3 * sizeof(float) * (size_t)W * H);
+        if (e == cudaSuccess) e = PadTexels(rgb, (size_t)W * H, env, ctx->stream);
+    }
+    for (uint32_t t = 0; anyTex && t < d->num_textures && e == cudaSuccess; t++) {
+        const pt_texture& X = d->textures[t];
+        const size_t n = (size_t)X.width * X.height;
+        const float* rgb = (const float*)lift(X.rgb, 3 * sizeof(float) * n);
+        if (e == cudaSuccess) e = PadTexels(rgb, n, texels + texInfo[t].x, ctx->stream);
+    }
+    if (e != cudaSuccess) {
+        cudaStreamSynchronize(ctx->stream);
+        for (auto& b : s.buffers) Free(ctx, b);
+        return e == cudaErrorMemoryAllocation ? Fail(ctx, PT_ERR_OUT_OF_MEMORY, "scene upload: allocation failed")
+                                              : CudaFail(ctx, e, "scene upload");
+    }
+    D.wide = D.nodes + wideOffset;
     D.numNodes = T > 0 ? (int)bvh.nodes.size() : 0;
-    D.numWide = (int)(wide.size() / (kWideFloats / 4));
+    D.numWide = (int)(wideF.size() / kWideFloats);
     D.numTris = T;
     D.numMats = (int)d->num_materials;
     D.numLights = (int)d->num_lights;
@@ -745,7 +720,7 @@ int pt_scene_upload(pt_context* ctx, const pt_scene_desc* d, pt_scene_id* out) {
     for (int a = 0; a < 3; a++) D.envBase[a] = d->env_base_color[a];
     D.envRot = d->env_z_rotation;
     D.lightPdfArea = 1.0f / sumArea;
-    const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
         for (auto& b : s.buffers) Free(ctx, b);
         return CudaFail(ctx, e, "scene upload");
