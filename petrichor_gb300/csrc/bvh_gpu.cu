@@ -581,9 +581,11 @@ template <int kN, int kItems>
 __global__ void __launch_bounds__(kN / kItems) BlockSortKernel(const int* __restrict__ count, int cap,
                                                                const int4* __restrict__ list, float* __restrict__ key,
                                                                int* __restrict__ ids, int2* __restrict__ heap,
-                                                               Counters* cnt, int heapCap) {
+                                                               BlockLists bl, Counters* cnt, int heapCap) {
     using Shared = BlockSortShared<kN, kItems>;
     constexpr int kT = Shared::kThreadsB;
+    // a subrange that fits the next smaller class goes there, where a block's round costs less
+    constexpr int kHandOff = kN == BlockSortMax(2) ? BlockSortMax(1) : kN == BlockSortMax(1) ? BlockSortMax(0) : 0;
     extern __shared__ __align__(16) char raw[];
     Shared& m = *reinterpret_cast<Shared*>(raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -711,6 +713,8 @@ __global__ void __launch_bounds__(kN / kItems) BlockSortKernel(const int* __rest
                             const int h = atomicAdd(&cnt->heap, 1);
                             if (h < heapCap) heap[h] = make_int2(base + lo[c], base + hi[c]);
                             else atomicOr(&cnt->error, kErrCapacity);
+                        } else if (len <= kHandOff) {
+                            PushBlockRange(bl, cnt, base + lo[c], base + hi[c], d);
                         } else {
                             const int x = atomicAdd(&m.nSeg[nxt], 1);
                             m.first[nxt][x] = (uint16_t)lo[c];
@@ -1163,7 +1167,7 @@ int LaunchBlockSort(int largest, const BlockLists& bl, float* key, int* ids, int
     const int bytes = (int)sizeof(BlockSortShared<kN, kItems>);
     if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     kernel<<<std::min(bl.cap[kClass], kClass == 2 ? 152 : kClass == 1 ? 1216 : 4864), kN / kItems, bytes, s>>>(
-      &cnt->block[kClass], bl.cap[kClass], bl.list[kClass], key, ids, heap, cnt, heapCap);
+      &cnt->block[kClass], bl.cap[kClass], bl.list[kClass], key, ids, heap, bl, cnt, heapCap);
     return 1;
 }
 
@@ -1342,9 +1346,10 @@ cudaError_t BuildBinnedSahDevice(const float* positions, int numVertices, const 
             }
             if (hc->error) break;
         }
-        launches += LaunchBlockSort<0>(largest, bl, key, ids, heap, cnt, heapCap, s);
-        launches += LaunchBlockSort<1>(largest, bl, key, ids, heap, cnt, heapCap, s);
+        // each class hands its small subranges to the next
         launches += LaunchBlockSort<2>(largest, bl, key, ids, heap, cnt, heapCap, s);
+        launches += LaunchBlockSort<1>(largest, bl, key, ids, heap, cnt, heapCap, s);
+        launches += LaunchBlockSort<0>(largest, bl, key, ids, heap, cnt, heapCap, s);
         HeapSortKernel<<<64, 64, 0, s>>>(cnt, heapCap, heap, key, ids);
         InsertionKernel<<<std::min(Blocks(smallCap), 1024), kThreads, 0, s>>>(cnt, smallCap, small, key, ids);
         // bins and the SAH split of every active node
