@@ -102,72 +102,6 @@ __global__ void PrimKernel(const float* __restrict__ P, const int32_t* __restric
     ids[t] = t;
 }
 
-// ---------------------------------------------------------------- prefix sum (int2)
-// Exclusive prefix sum of n int2 values, 1024 per block; block totals are summed
-// recursively and added back.
-__global__ void ScanBlocks(const int2* __restrict__ in, int2* __restrict__ out,
-                           int2* __restrict__ blockSums, int n) {
-    __shared__ int2 warpSums[kThreads / 32];
-    const int base = (blockIdx.x * kThreads + threadIdx.x) * kScanItems;
-    int2 v[kScanItems];
-    int2 sum = make_int2(0, 0);
-    for (int j = 0; j < kScanItems; j++) {
-        v[j] = base + j < n ? in[base + j] : make_int2(0, 0);
-        sum.x += v[j].x;
-        sum.y += v[j].y;
-    }
-    // inclusive scan of the per-thread sums within the warp
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int2 inc = sum;
-    for (int d = 1; d < 32; d <<= 1) {
-        const int x = __shfl_up_sync(kFull, inc.x, d), y = __shfl_up_sync(kFull, inc.y, d);
-        if (lane >= d) inc.x += x, inc.y += y;
-    }
-    if (lane == 31) warpSums[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-        int2 w = lane < kThreads / 32 ? warpSums[lane] : make_int2(0, 0);
-        for (int d = 1; d < kThreads / 32; d <<= 1) {
-            const int x = __shfl_up_sync(kFull, w.x, d), y = __shfl_up_sync(kFull, w.y, d);
-            if (lane >= d) w.x += x, w.y += y;
-        }
-        if (lane < kThreads / 32) warpSums[lane] = w;
-    }
-    __syncthreads();
-    int2 run = make_int2(inc.x - sum.x, inc.y - sum.y);
-    if (warp > 0) run.x += warpSums[warp - 1].x, run.y += warpSums[warp - 1].y;
-    for (int j = 0; j < kScanItems; j++) {
-        if (base + j < n) out[base + j] = run;
-        run.x += v[j].x;
-        run.y += v[j].y;
-    }
-    if (threadIdx.x == kThreads - 1 && blockSums) blockSums[blockIdx.x] = run;
-}
-
-__global__ void AddBlockOffsets(int2* __restrict__ out, const int2* __restrict__ offsets, int n) {
-    const int base = (blockIdx.x * kThreads + threadIdx.x) * kScanItems;
-    const int2 o = offsets[blockIdx.x];
-    for (int j = 0; j < kScanItems; j++)
-        if (base + j < n) out[base + j].x += o.x, out[base + j].y += o.y;
-}
-
-struct ScanScratch {
-    std::vector<int2*> levels;  // block sums of each recursion level
-    std::vector<int> sizes;
-};
-
-void ExclusiveScan(const int2* in, int2* out, int n, const ScanScratch& sc, int level,
-                   cudaStream_t s) {
-    const int per = kThreads * kScanItems;
-    const int nb = (n + per - 1) / per;
-    int2* sums = nb > 1 ? sc.levels[level] : nullptr;
-    ScanBlocks<<<nb, kThreads, 0, s>>>(in, out, sums, n);
-    if (nb > 1) {
-        ExclusiveScan(sums, sums, nb, sc, level + 1, s);
-        AddBlockOffsets<<<nb, kThreads, 0, s>>>(out, sums, n);
-    }
-}
-
 // ---------------------------------------------------------------- run reductions
 // Positions are reduced into per-target accumulators where consecutive positions
 // mostly share a target (a node, or a node's bin). Each thread folds kRun
@@ -349,34 +283,102 @@ __device__ __forceinline__ int MedianPlace(const float* key, int f, int l) {
 
 // __unguarded_partition_pivot's pivot: std::__move_median_to_first(first, first + 1,
 // mid, last - 1).
-__global__ void PivotKernel(int nSeg, SegList segs, float* __restrict__ key, int* __restrict__ ids) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nSeg) return;
-    const int f = segs.first[s], l = segs.last[s];
-    const int m = MedianPlace(key, f, l);
-    SwapAt(key, ids, f, m);
+__device__ __forceinline__ void StartRange(const SegList& segs, int s, float* key, int* ids) {
+    const int f = segs.first[s];
+    SwapAt(key, ids, f, MedianPlace(key, f, segs.last[s]));
     segs.pivot[s] = key[f];
     segs.K[s] = INT_MAX;
 }
-
-// flags.x: position of [f+1, l) with !(key < pivot); flags.y: position of [f, l) with
-// !(pivot < key). Entry T stays zero so the prefix sum holds the totals.
-__global__ void FlagsKernel(int T, const int* __restrict__ seg, SegList segs,
-                            const float* __restrict__ key, int2* __restrict__ flags) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > T) return;
-    int2 f = make_int2(0, 0);
-    const int s = i < T ? seg[i] : -1;
-    if (s >= 0) {
-        const float pv = segs.pivot[s], k = key[i];
-        f.x = (i > segs.first[s] && !(k < pv)) ? 1 : 0;
-        f.y = !(pv < k) ? 1 : 0;
-    }
-    flags[i] = f;
+__global__ void PivotKernel(int nSeg, SegList segs, float* __restrict__ key, int* __restrict__ ids) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < nSeg) StartRange(segs, s, key, ids);
 }
 
+// Exclusive prefix sums of two flags per position (x: position of [f+1, l) with
+// !(key < pivot); y: position of [f, l) with !(pivot < key)) over [0, T], so entry T holds the
+// totals: within blocks of kScanSpan positions, whose totals ScanTopKernel turns into their
+// offsets. ScanAt adds the two.
+constexpr int kScanSpan = kThreads * kScanItems;
+__global__ void __launch_bounds__(kThreads) ScanFlagsKernel(int T, const int* __restrict__ seg, SegList segs,
+                                                            const float* __restrict__ key, int2* __restrict__ pre,
+                                                            int2* __restrict__ blockSums) {
+    __shared__ int2 warpSums[kThreads / 32];
+    const int base = blockIdx.x * kScanSpan + threadIdx.x * kScanItems;
+    int2 v[kScanItems];
+    int2 sum = make_int2(0, 0);
+    for (int j = 0; j < kScanItems; j++) {
+        const int i = base + j;
+        v[j] = make_int2(0, 0);
+        const int s = i < T ? seg[i] : -1;
+        if (s >= 0) {
+            const float pv = segs.pivot[s], k = key[i];
+            v[j].x = (i > segs.first[s] && !(k < pv)) ? 1 : 0;
+            v[j].y = !(pv < k) ? 1 : 0;
+        }
+        sum.x += v[j].x;
+        sum.y += v[j].y;
+    }
+    // inclusive scan of the per-thread sums within the warp
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int2 inc = sum;
+    for (int d = 1; d < 32; d <<= 1) {
+        const int x = __shfl_up_sync(kFull, inc.x, d), y = __shfl_up_sync(kFull, inc.y, d);
+        if (lane >= d) inc.x += x, inc.y += y;
+    }
+    if (lane == 31) warpSums[warp] = inc;
+    __syncthreads();
+    int2 run = make_int2(inc.x - sum.x, inc.y - sum.y);
+    for (int w = 0; w < warp; w++) run.x += warpSums[w].x, run.y += warpSums[w].y;
+    for (int j = 0; j < kScanItems; j++) {
+        if (base + j <= T) pre[base + j] = run;
+        run.x += v[j].x;
+        run.y += v[j].y;
+    }
+    if (threadIdx.x == kThreads - 1) blockSums[blockIdx.x] = run;
+}
+
+// One block: exclusive scan of the n block totals in place; the next round's subrange count
+// starts at zero.
+__global__ void __launch_bounds__(1024) ScanTopKernel(int n, int2* __restrict__ sums, Counters* cnt) {
+    __shared__ int2 warpSums[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) cnt->segs = 0;
+    int2 carry = make_int2(0, 0);
+    for (int b = 0; b < n; b += 1024) {
+        const int i = b + threadIdx.x;
+        const int2 v = i < n ? sums[i] : make_int2(0, 0);
+        int2 inc = v;
+        for (int d = 1; d < 32; d <<= 1) {
+            const int x = __shfl_up_sync(kFull, inc.x, d), y = __shfl_up_sync(kFull, inc.y, d);
+            if (lane >= d) inc.x += x, inc.y += y;
+        }
+        if (lane == 31) warpSums[warp] = inc;
+        __syncthreads();
+        int2 w = warpSums[lane];
+        for (int d = 1; d < 32; d <<= 1) {
+            const int x = __shfl_up_sync(kFull, w.x, d), y = __shfl_up_sync(kFull, w.y, d);
+            if (lane >= d) w.x += x, w.y += y;
+        }
+        const int bx = __shfl_sync(kFull, w.x, max(warp - 1, 0)), by = __shfl_sync(kFull, w.y, max(warp - 1, 0));
+        if (i < n)
+            sums[i] = make_int2(carry.x + (warp ? bx : 0) + inc.x - v.x, carry.y + (warp ? by : 0) + inc.y - v.y);
+        carry.x += __shfl_sync(kFull, w.x, 31);
+        carry.y += __shfl_sync(kFull, w.y, 31);
+        __syncthreads();
+    }
+}
+
+struct Prefix {
+    const int2* pre;
+    const int2* offset;
+    __device__ __forceinline__ int2 operator[](int i) const {
+        const int2 a = pre[i], b = offset[i / kScanSpan];
+        return make_int2(a.x + b.x, a.y + b.y);
+    }
+};
+
 __global__ void RanksKernel(int T, const int* __restrict__ seg, SegList segs,
-                            const int2* __restrict__ pre, int* __restrict__ lpos,
+                            Prefix pre, int* __restrict__ lpos,
                             int* __restrict__ rpos) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int s = i < T ? seg[i] : -1;
@@ -403,7 +405,7 @@ __global__ void RanksKernel(int T, const int* __restrict__ seg, SegList segs,
 }
 
 __global__ void SwapKernel(int T, const int* __restrict__ seg, SegList segs,
-                           const int2* __restrict__ pre, const int* __restrict__ lpos,
+                           Prefix pre, const int* __restrict__ lpos,
                            const int* __restrict__ rpos, float* __restrict__ key,
                            int* __restrict__ ids, Counters* cnt) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -433,7 +435,8 @@ __global__ void SwapKernel(int T, const int* __restrict__ seg, SegList segs,
 // Children of each partitioned subrange, as __introsort_loop continues with them:
 // both halves with the decremented depth; more than 16 elements and no depth left:
 // heapsort; 16 or fewer: left to the final insertion sort.
-__global__ void SplitSegsKernel(int nSeg, SegList segs, SegList next, int2* __restrict__ small,
+__global__ void SplitSegsKernel(int nSeg, SegList segs, SegList next, float* __restrict__ key,
+                                int* __restrict__ ids, int2* __restrict__ small,
                                 int2* __restrict__ heap, BlockLists bl, Counters* cnt, int segCap,
                                 int smallCap, int heapCap) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -455,6 +458,7 @@ __global__ void SplitSegsKernel(int nSeg, SegList segs, SegList next, int2* __re
                     next.first[x] = lo[c];
                     next.last[x] = hi[c];
                     next.depth[x] = d;
+                    StartRange(next, x, key, ids);
                     idx[c] = x;
                 } else {
                     atomicOr(&cnt->error, kErrCapacity);
@@ -1089,7 +1093,7 @@ struct BuildArrays {
     int* ids;
     float* key;
     int *nodeOf, *seg;
-    int2 *flags, *pre;
+    int2 *pre, *spanSums;
     int *lpos, *rpos;
     TempNodes tn;
     LevelNodes lv[2];
@@ -1106,7 +1110,6 @@ struct BuildArrays {
     Counters* cnt;
     int *ic, *index, *rank;
     OutNode* outNodes;
-    ScanScratch scan;
     void Carve(Arena& ar, int T, int numVertices, int nodeCap, int activeCap, int segCap, int smallCap, int heapCap) {
         const size_t t = (size_t)T;
         dPos = ar.Get<float>(3 * (size_t)numVertices);
@@ -1117,8 +1120,8 @@ struct BuildArrays {
         key = ar.Get<float>(t);
         nodeOf = ar.Get<int>(t);
         seg = ar.Get<int>(t);
-        flags = ar.Get<int2>(t + 1);
         pre = ar.Get<int2>(t + 1);
+        spanSums = ar.Get<int2>(t / kScanSpan + 1);
         lpos = ar.Get<int>(t);
         rpos = ar.Get<int>(t);
         tn = TempNodes{ar.Get<int>(nodeCap), ar.Get<int>(nodeCap), ar.Get<int>(nodeCap),
@@ -1148,12 +1151,6 @@ struct BuildArrays {
         index = ar.Get<int>(nodeCap);
         rank = ar.Get<int>(nodeCap);
         outNodes = ar.Get<OutNode>(nodeCap);
-        scan = ScanScratch{};
-        for (long long n = (long long)t + 1; n > kThreads * kScanItems;) {
-            n = (n + kThreads * kScanItems - 1) / (kThreads * kScanItems);
-            scan.levels.push_back(ar.Get<int2>(n));
-            scan.sizes.push_back((int)n);
-        }
     }
 };
 
@@ -1221,7 +1218,7 @@ cudaError_t BuildBinnedSahDevice(const float* positions, int numVertices, const 
     auto& key = arrays.key;
     auto& nodeOf = arrays.nodeOf;
     auto& seg = arrays.seg;
-    auto& flags = arrays.flags;
+    auto& spanSums = arrays.spanSums;
     auto& pre = arrays.pre;
     auto& lpos = arrays.lpos;
     auto& rpos = arrays.rpos;
@@ -1246,7 +1243,6 @@ cudaError_t BuildBinnedSahDevice(const float* positions, int numVertices, const 
     auto& index = arrays.index;
     auto& rank = arrays.rank;
     auto& outNodes = arrays.outNodes;
-    auto& scan = arrays.scan;
     struct HostFree {
         Counters* p;
         ~HostFree() { cudaFreeHost(p); }
@@ -1326,20 +1322,23 @@ cudaError_t BuildBinnedSahDevice(const float* positions, int numVertices, const 
         if (largest > BlockSortMax(2)) {
             if ((e = fetch()) != cudaSuccess) return e;
             int nSeg = hc->segs, sc = 0;
+            bool fresh = true;
             while (nSeg > 0 && hc->error == 0) {
                 rounds++;
                 SegList& S = sl[sc];
                 SegList& X = sl[sc ^ 1];
-                PivotKernel<<<Blocks(nSeg), kThreads, 0, s>>>(nSeg, S, key, ids);
-                FlagsKernel<<<Blocks(T + 1), kThreads, 0, s>>>(T, seg, S, key, flags);
-                ExclusiveScan(flags, pre, T + 1, scan, 0, s);
-                RanksKernel<<<Blocks(T), kThreads, 0, s>>>(T, seg, S, pre, lpos, rpos);
-                SwapKernel<<<Blocks(T), kThreads, 0, s>>>(T, seg, S, pre, lpos, rpos, key, ids, cnt);
-                ResetCounters<<<1, 1, 0, s>>>(cnt, 1, 0, 0, 0);
-                SplitSegsKernel<<<Blocks(nSeg), kThreads, 0, s>>>(nSeg, S, X, small, heap, bl, cnt, segCap,
+                if (fresh) PivotKernel<<<Blocks(nSeg), kThreads, 0, s>>>(nSeg, S, key, ids);
+                fresh = false;  // later subranges get their pivots where they are split off
+                const int spans = Blocks((long long)T + 1, kScanSpan);
+                const Prefix sums{pre, spanSums};
+                ScanFlagsKernel<<<spans, kThreads, 0, s>>>(T, seg, S, key, pre, spanSums);
+                ScanTopKernel<<<1, 1024, 0, s>>>(spans, spanSums, cnt);
+                RanksKernel<<<Blocks(T), kThreads, 0, s>>>(T, seg, S, sums, lpos, rpos);
+                SwapKernel<<<Blocks(T), kThreads, 0, s>>>(T, seg, S, sums, lpos, rpos, key, ids, cnt);
+                SplitSegsKernel<<<Blocks(nSeg), kThreads, 0, s>>>(nSeg, S, X, key, ids, small, heap, bl, cnt, segCap,
                                                                  smallCap, heapCap);
                 ResegKernel<<<Blocks(T), kThreads, 0, s>>>(T, seg, S);
-                launches += 8 + 2 * (int)scan.levels.size() + 1;
+                launches += 6;
                 if ((e = fetch()) != cudaSuccess) return e;
                 nSeg = hc->segs;
                 sc ^= 1;

@@ -54,3 +54,9 @@ def test_depth_budget_runs_out(gpu_ctx, tmp_path, n):
     keys = subprocess.run([exe, str(n)], capture_output=True, text=True, check=True).stdout.split()
     stats = _same(gpu_ctx, *_triangles(np.array(keys, np.int64)))
     assert stats.heapsorts > 0
+
+
+def test_more_positions_than_one_block_scans(gpu_ctx):
+    """1.1M triangles: the partition rounds' prefix sums have more spans than ScanTopKernel's
+    block has threads."""
+    _same(gpu_ctx, *_triangles(np.random.default_rng(2).integers(0, 1 << 20, 1_100_000)))
