@@ -14,6 +14,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "env_row.h"
 #include "pt_layout.h"
 
 namespace ptg {
@@ -466,7 +467,8 @@ __device__ __forceinline__ void EnvSampleSearch(const DevScene& S, float r0, flo
 // form, evaluated here bit for bit:
 //   row search: every compared midpoint v is an odd multiple of 2^-k with k <= log2 H,
 //     so y = v H is an integer, the lerp weight is exactly 0 and the table value is
-//     cdf1D[y] = (y + 1) / H = v + 1/H exactly: the comparisons reduce to v + 1/H - r0;
+//     cdf1D[y] = (y + 1) / H = v + 1/H exactly: the comparisons reduce to v + 1/H - r0, and
+//     the search to one expression (EnvRow);
 //   column search: for u = 2^-k (k <= log2 W) and the row found above (a multiple of
 //     1/(2H)), every bilinear weight is 0, 1/2 or 1 and the unloaded-table read is
 //     exactly 1, so 1 - r1 >= 0 at every step: u shrinks to 0.5 / W whatever r1 is;
@@ -474,17 +476,10 @@ __device__ __forceinline__ void EnvSampleSearch(const DevScene& S, float r0, flo
 template <class M>
 __device__ __forceinline__ V3 EnvSample(const DevScene& S, float r0, float r1, float& pdf) {
     const int W = S.envW, H = S.envH;
-    const float tw = 1.0f / W, th = 1.0f / H;
-    float u0, v0 = 0.0f, v1 = 1.0f;
+    const float tw = 1.0f / W;
+    float u0, v0;
     if (((W & (W - 1)) | (H & (H - 1))) == 0 && W <= (1 << 22) && H <= (1 << 22)) {
-        for (int it = 0; it < 64; it++) {
-            const float v = 0.5f * (v0 + v1);
-            const float diff = (v + th) - r0;
-            if (v1 - v0 <= th) { v0 = v1 = v; break; }
-            if (diff > 0) v1 = v;
-            else if (diff < 0) v0 = v;
-            else { v0 = v1 = v; break; }
-        }
+        v0 = EnvRow(r0, H);
         u0 = 0.5f * tw;
         pdf = 1.0f;
     } else {
