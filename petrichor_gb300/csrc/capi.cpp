@@ -22,6 +22,7 @@
 #include "bvh_builder.h"
 #include "bvh_gpu.h"
 #include "denoise.h"
+#include "env_row.h"
 #include "pt_kernels.h"
 #include "pt_layout.h"
 #include "context.h"
@@ -641,6 +642,10 @@ int pt_scene_upload(pt_context* ctx, const pt_scene_desc* d, pt_scene_id* out) {
     SceneGpu& s = *sg;
     DevScene& D = s.dev;
     float4 *tree = nullptr, *tris = nullptr, *shade = nullptr, *env = nullptr, *texels = nullptr, *uvs = nullptr;
+    // the sampler's outcomes are tabled for maps it has a closed form for (EnvSample)
+    const bool envTabled = W > 0 && (W & (W - 1)) == 0 && (H & (H - 1)) == 0 && W <= (1 << 22) && H <= kEnvTableRows;
+    float4 *envTable = nullptr, *envTableExact = nullptr;
+    const size_t envTableBytes = 2 * (size_t)H * 2 * sizeof(float4);
     const size_t slot3 = 3 * sizeof(float4);
     const bool withUV = anyUV || anyTex;
     if ((rc = SceneBuffer(ctx, s, wideOffset * sizeof(float4) + wideF.size() * sizeof(float), &tree)) != PT_OK ||
@@ -648,6 +653,8 @@ int pt_scene_upload(pt_context* ctx, const pt_scene_desc* d, pt_scene_id* out) {
         (rc = SceneBuffer(ctx, s, (size_t)T * slot3, &shade)) != PT_OK ||
         (rc = Upload(ctx, s, mats, &D.mats)) != PT_OK || (rc = Upload(ctx, s, lights, &D.lights)) != PT_OK ||
         (rc = SceneBuffer(ctx, s, std::max<size_t>((size_t)W * H, 1) * sizeof(float4), &env)) != PT_OK ||
+        (envTabled && (rc = SceneBuffer(ctx, s, envTableBytes, &envTable)) != PT_OK) ||
+        (envTabled && (rc = SceneBuffer(ctx, s, envTableBytes, &envTableExact)) != PT_OK) ||
         (anyTex && (rc = SceneBuffer(ctx, s, std::max<size_t>(numTexels, 1) * sizeof(float4), &texels)) != PT_OK) ||
         (anyTex && (rc = Upload(ctx, s, texInfo, &D.texInfo)) != PT_OK) ||
         (withUV && (rc = SceneBuffer(ctx, s, (size_t)std::max(T, 1) * slot3, &uvs)) != PT_OK)) {
@@ -720,7 +727,13 @@ int pt_scene_upload(pt_context* ctx, const pt_scene_desc* d, pt_scene_id* out) {
     for (int a = 0; a < 3; a++) D.envBase[a] = d->env_base_color[a];
     D.envRot = d->env_z_rotation;
     D.lightPdfArea = 1.0f / sumArea;
-    e = cudaStreamSynchronize(ctx->stream);
+    if (envTabled) {
+        e = FillEnvTable(D, envTable, ctx->stream);
+        if (e == cudaSuccess) e = FillEnvTableExact(D, envTableExact, ctx->stream);
+        D.envTable = envTable;
+        D.envTableExact = envTableExact;
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
         for (auto& b : s.buffers) Free(ctx, b);
         return CudaFail(ctx, e, "scene upload");

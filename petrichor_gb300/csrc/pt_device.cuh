@@ -85,6 +85,7 @@ __device__ __forceinline__ V3 LoadV3(const float* p) { return V3(p[0], p[1], p[2
 
 // ---------------------------------------------------------------- math policies
 struct ExactMath {
+    static __device__ __forceinline__ const float4* EnvTable(const DevScene& S) { return S.envTableExact; }
     static __device__ __forceinline__ float Cos(float x) { return (float)cos((double)x); }
     static __device__ __forceinline__ float Sin(float x) { return (float)sin((double)x); }
     static __device__ __forceinline__ float Acos(float x) { return (float)acos((double)x); }
@@ -128,6 +129,7 @@ struct ExactMath {
 // large-argument reduction, and the shade kernel's code stays small enough for the
 // instruction cache. They agree with sinf/cosf to a few ulps.
 struct FastMath {
+    static __device__ __forceinline__ const float4* EnvTable(const DevScene& S) { return S.envTable; }
     static __device__ __forceinline__ float Cos(float x) { return cospif(x * kInvPi); }
     static __device__ __forceinline__ float Sin(float x) { return sinpif(x * kInvPi); }
     // clamped: directions normalised with approximate division may reach |z| > 1
@@ -461,6 +463,15 @@ __device__ __forceinline__ void EnvSampleSearch(const DevScene& S, float r0, flo
         pdf = py * UnloadedTableBilinearX(u0, v0, W, H);
     }
 }
+// The direction of map coordinates (u0, v0).
+template <class M>
+__device__ __forceinline__ V3 EnvDirection(const DevScene& S, float u0, float v0) {
+    const float theta = v0 * kPi;
+    const float phi = 2.0f * kPi * (1.0f - u0) + S.envRot;
+    // ONB(UnitZ, UnitX).GetDir(theta, phi): u = X, v = Y, w = Z
+    const float cx = M::SinCos(theta, phi), cy = M::SinSin(theta, phi), cz = M::Cos(theta);
+    return cx * V3(1.f, 0.f, 0.f) + cy * V3(0.f, 1.f, 0.f) + cz * V3(0.f, 0.f, 1.f);
+}
 // Environment::ImportanceSampling (Environment.cpp:130-220)
 //
 // When W and H are powers of two (all configured maps) both searches have a closed
@@ -485,11 +496,31 @@ __device__ __forceinline__ V3 EnvSample(const DevScene& S, float r0, float r1, f
     } else {
         EnvSampleSearch(S, r0, r1, u0, v0, pdf);
     }
-    const float theta = v0 * kPi;
-    const float phi = 2.0f * kPi * (1.0f - u0) + S.envRot;
-    // ONB(UnitZ, UnitX).GetDir(theta, phi): u = X, v = Y, w = Z
-    const float cx = M::SinCos(theta, phi), cy = M::SinSin(theta, phi), cz = M::Cos(theta);
-    return cx * V3(1.f, 0.f, 0.f) + cy * V3(0.f, 1.f, 0.f) + cz * V3(0.f, 0.f, 1.f);
+    return EnvDirection<M>(S, u0, v0);
+}
+// The sample with its radiance. A power-of-two map's outcomes are read from the scene's table
+// (EnvTableEntry formed them with the same functions): one 32-byte read instead of the sines
+// and cosines of the direction, the arc functions of its lookup and four texels.
+template <class M>
+__device__ __forceinline__ V3 EnvSampleLit(const DevScene& S, float r0, float r1, float& pdf, V3& li) {
+    const float4* table = M::EnvTable(S);
+    if (table) {
+        const int e = (int)(2.0f * EnvRowAt(r0, S.envH));
+        const float4 d = __ldg(table + 2 * e), c = __ldg(table + 2 * e + 1);
+        pdf = 1.0f;
+        li = V3(c.x, c.y, c.z);
+        return V3(d.x, d.y, d.z);
+    }
+    const V3 sd = EnvSample<M>(S, r0, r1, pdf);
+    li = EnvColor<M>(S, sd);
+    return sd;
+}
+template <class M>
+__device__ __forceinline__ void EnvTableEntry(const DevScene& S, int e, float4* table) {
+    const V3 d = EnvDirection<M>(S, 0.5f * (1.0f / S.envW), 0.5f * (float)e * (1.0f / (float)S.envH));
+    const V3 c = EnvColor<M>(S, d);
+    table[2 * e] = make_float4(d.x, d.y, d.z, 0.0f);
+    table[2 * e + 1] = make_float4(c.x, c.y, c.z, 0.0f);
 }
 // Environment::GetImportanceSamplingPDF (Environment.cpp:222-244)
 template <class M>

@@ -29,6 +29,11 @@ cudaError_t LaunchReplay(const DevScene& S, const DevCamera& C, const DevSetting
                          int* stackScratch, int* status, int tileBegin, int tileEnd,
                          cudaStream_t stream);
 
+// The environment sampler's outcomes of a scene whose map is in place (DevScene::envTable and
+// envTableExact, 2 envH entries of two float4).
+cudaError_t FillEnvTable(const DevScene& S, float4* table, cudaStream_t stream);
+cudaError_t FillEnvTableExact(const DevScene& S, float4* table, cudaStream_t stream);
+
 // AOV pass (0 UV, 1 denoising albedo, 2 denoising normal) of tiles [tileBegin, tileEnd):
 // one warp per tile with the reference's per-tile stream; dspp = numSppForDenoising.
 cudaError_t LaunchAov(const DevScene& S, const DevCamera& C, const DevSettings& st, int aov,

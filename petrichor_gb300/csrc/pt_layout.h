@@ -91,6 +91,11 @@ struct DevScene {
     // {keep threshold, alias index (bits), pdf over (u, v), 0}; nullptr: the reference's
     // sampler
     const float4* envAlias;
+    // The reference sampler's outcomes (power-of-two maps of up to kEnvTableRows rows), entry
+    // 2 v H for the sampled v: {direction.xyz, 0}, {radiance.rgb, 0}; in the throughput path's
+    // arithmetic and in the replay's. nullptr: formed per sample.
+    const float4* envTable;
+    const float4* envTableExact;
     int32_t numNodes, numTris, numMats, numLights;
     int32_t envW, envH, envValid, stackDepth;  // stackDepth: max traversal stack entries
     float envBase[3], envRot;

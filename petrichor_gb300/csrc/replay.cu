@@ -278,7 +278,8 @@ __device__ V3 ReplayLight(const DevScene& S, const Shading& si, const DevMateria
         float r0, r1;
         s2.Next(r0, r1);
         float pdfuv = 0.0f;
-        const V3 sd = EnvSample<ExactMath>(S, r0, r1, pdfuv);
+        V3 li;
+        const V3 sd = EnvSampleLit<ExactMath>(S, r0, r1, pdfuv, li);
         const V3 eo = si.pos + kEps * copysignf(1.0f, dt) * si.n;
         float d;
         if (TraverseWarp(S, eo, sd, 0.0f, kFltMax, d, stack, status) < 0) {
@@ -286,7 +287,6 @@ __device__ V3 ReplayLight(const DevScene& S, const Shading& si, const DevMateria
             const float sn = sqrtf(SMax(0.0f, 1.0f - c * c));
             const float pB = 2.0f * kPi * kPi * sn * BsdfPdf<ExactMath>(M, ray.d, sd, nb);
             const float mis = pdfuv * pdfuv / (pdfuv * pdfuv + pB * pB);
-            const V3 li = EnvColor<ExactMath>(S, sd);
             const V3 f = BxDF<ExactMath>(M, ray.d, sd, nb);
             lc = lc + mis * ray.T * (li * f * sn * c * 2.0f * kPi * kPi) / pdfuv;
         }
@@ -510,6 +510,15 @@ cudaError_t LaunchAov(const DevScene& S, const DevCamera& C, const DevSettings& 
     if (n <= 0) return cudaSuccess;
     AovKernel<<<n, 32, 0, stream>>>(S, C, st, aov, dspp, film, stackScratch,
                                                               status, tileBegin, tileEnd);
+    return cudaGetLastError();
+}
+
+__global__ void EnvTableExactKernel(DevScene S, float4* __restrict__ table) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < 2 * S.envH) EnvTableEntry<ExactMath>(S, e, table);
+}
+cudaError_t FillEnvTableExact(const DevScene& S, float4* table, cudaStream_t stream) {
+    EnvTableExactKernel<<<(2 * S.envH + 31) / 32, 32, 0, stream>>>(S, table);
     return cudaGetLastError();
 }
 

@@ -34,7 +34,7 @@ namespace ptg {
 #define PT_TRACE_MIN_BLOCKS 7
 #endif
 // Resident blocks per SM of the shade stage, and its grid (see ShadeKernel).
-constexpr int kShadeBlocks = 5;
+constexpr int kShadeBlocks = 6;
 
 enum : int { kFlagNoSignCheck = 1 };
 enum : int { kShadowEnv = 0, kShadowArea = 1 };
@@ -695,14 +695,15 @@ __device__ __forceinline__ void ShadeOne(const DevJob& J, int path, V3 o, V3 d, 
                         float e0, e1;
                         rng.Next(e0, e1);
                         float pdfuv = 0.0f;
-                        V3 sd;
+                        V3 sd, li;
                         const bool alias = S.envAlias != nullptr;
                         if (alias) {
                             float j0, j1;
                             rng.Next(j0, j1);
                             sd = EnvSampleAlias<FastMath>(S, e0, e1, j0, j1, pdfuv);
+                            li = EnvColor<FastMath>(S, sd);
                         } else {
-                            sd = EnvSample<FastMath>(S, e0, e1, pdfuv);
+                            sd = EnvSampleLit<FastMath>(S, e0, e1, pdfuv, li);
                         }
                         const float c = fabsf(FastMath::Dot(sd, si.n));
                         // sin theta of the (u, v) -> solid angle Jacobian: the map's polar
@@ -711,7 +712,6 @@ __device__ __forceinline__ void ShadeOne(const DevJob& J, int path, V3 o, V3 d, 
                         const float sn = sqrtf(SMax(0.0f, 1.0f - zc * zc));
                         const float pB = 2.0f * kPi * kPi * sn * BsdfPdf<FastMath>(M, d, sd, nb);
                         const float mis = pdfuv * pdfuv / (pdfuv * pdfuv + pB * pB);
-                        const V3 li = EnvColor<FastMath>(S, sd);
                         const V3 f = BxDF<FastMath>(M, d, sd, nb);
                         const V3 contrib = mis * in.T * (li * f * sn * c * 2.0f * kPi * kPi) / pdfuv;
                         if (contrib.x != 0.0f || contrib.y != 0.0f || contrib.z != 0.0f) {
@@ -788,8 +788,10 @@ __device__ __forceinline__ void CopyAsyncWait() { asm volatile("cp.async.wait_al
 // counters in one instruction when all its lanes are done (two lanes, one counter each),
 // and a path that ends before any next-event ray could add to it writes its radiance
 // without reading it. Shade stage of the 1.0M-triangle 1080p frame: 13.78 ms with loads at
-// the start and two appends a step; one append 12.50, entries staged ahead 11.33, and at
-// 5 blocks of 102 registers instead of 4 10.21 ms (6 blocks 10.18, 7 11.29, 8 11.57).
+// the start and two appends a step; one append 12.50, entries staged ahead 11.33, 5 blocks
+// instead of 4 10.21, short first entries 9.90, the environment row in closed form 8.82, and
+// the environment sample from its table 7.79 (4, 5, 6, 7 blocks: 8.81, 7.78, 7.72, 8.00; 4K
+// terrain 4.27, 3.83, 3.77, 3.68).
 // kFirst: the queue is raygen's, short entries (RaygenKernel); every path's radiance is
 // written here.
 template <int kInteg, bool kFirst>
@@ -1190,6 +1192,15 @@ __global__ void FinalizeKernel(const DevJob* __restrict__ jobs, const int* __res
         J.film[3 * i + 1] = a.y / inv;
         J.film[3 * i + 2] = a.z / inv;
     }
+}
+
+__global__ void EnvTableKernel(DevScene S, float4* __restrict__ table) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < 2 * S.envH) EnvTableEntry<FastMath>(S, e, table);
+}
+cudaError_t FillEnvTable(const DevScene& S, float4* table, cudaStream_t stream) {
+    EnvTableKernel<<<(2 * S.envH + 127) / 128, 128, 0, stream>>>(S, table);
+    return cudaGetLastError();
 }
 
 struct RayBatchQueue {
