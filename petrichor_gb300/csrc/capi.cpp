@@ -1119,7 +1119,10 @@ int pt_trace_closest(pt_context* ctx, pt_scene_id scene, int32_t n, const float*
         return Fail(ctx, PT_ERR_INVALID_ARG, "bad ray buffers");
     int rc = SetDevice(ctx);
     if (rc != PT_OK) return rc;
+    const bool fresh = !ctx->status.ptr;
     if ((rc = Alloc(ctx, ctx->status, 16)) != PT_OK) return rc;
+    // the first word is the status of tile renders, read back after every render
+    if (fresh) cudaMemset(ctx->status.ptr, 0, 16);
     const cudaError_t e = LaunchTraceClosest(it->second->dev, n, rays, distMin, distMax, tri, dist,
                                              (int*)ctx->status.ptr + 1,
                                              stream ? (cudaStream_t)stream : ctx->stream);
