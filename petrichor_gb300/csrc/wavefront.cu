@@ -111,11 +111,12 @@ __device__ __forceinline__ void SortPair(float& ta, int& ca, float& tb, int& cb)
 
 // Entries of the traversal stack kept in shared memory per thread; deeper ones go
 // to local memory. Shared entries are entry-major with one column per thread of
-// the 128-thread block, so a warp's accesses always fall in 32 distinct banks. 8 entries
-// leave more of the SM's memory to L1 and to the other stream's blocks than 12 or 16: a
-// 2.2M-triangle 4K terrain frame took 27.66, 27.89 and 27.91 ms.
+// the 128-thread block, so a warp's accesses always fall in 32 distinct banks. More entries
+// take from L1 and from the other stream's blocks: a 1.0M-triangle 1080p still took 40.01,
+// 39.85, 39.91 and 39.92 ms with 8, 10, 12 and 16, a 2.2M-triangle 4K terrain frame 23.54, 23.45,
+// 23.70 and 23.71 ms.
 #ifndef PT_SMEM_STACK
-#define PT_SMEM_STACK 8
+#define PT_SMEM_STACK 10
 #endif
 constexpr int kTraceBlock = 128;
 constexpr int kTraceWarps = kTraceBlock / 32;
