@@ -27,8 +27,8 @@
 namespace ptg {
 
 // Minimum resident blocks per SM requested from the register allocator for the
-// trace (extend/shadow) stages: 7 blocks of at most 72 registers; 8 of 64 (which spill), 6
-// and 5 measured 17.65, 17.30 and 17.85 ms against 16.90 for the closest hits of the
+// trace (extend/shadow) stages: 7 blocks of at most 72 registers (the closest-hit kernel
+// takes 64 of them, so 8 of its blocks are resident); 8 of 64 (the others spill), 6 and 5 measured 17.65, 17.30 and 17.85 ms against 16.90 for the closest hits of the
 // 1.0M-triangle 1080p frame.
 #ifndef PT_TRACE_MIN_BLOCKS
 #define PT_TRACE_MIN_BLOCKS 7
