@@ -707,6 +707,7 @@ int pt_scene_upload(pt_context* ctx, const pt_scene_desc* d, pt_scene_id* out) {
         if (e == cudaSuccess) e = PadTexels(rgb, n, texels + texInfo[t].x, ctx->stream);
     }
     if (e != cudaSuccess) {
+        cudaGetLastError();  // a failed allocation's error is not the next launch's
         cudaStreamSynchronize(ctx->stream);
         for (auto& b : s.buffers) Free(ctx, b);
         return e == cudaErrorMemoryAllocation ? Fail(ctx, PT_ERR_OUT_OF_MEMORY, "scene upload: allocation failed")
