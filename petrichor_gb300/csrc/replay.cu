@@ -14,7 +14,8 @@
 // are tested side by side. FP64 costs a warp the same with one active lane or 32.
 // One thread per tile, 32 diverging tiles to a warp, took 173.4 ms for a 256x256 2-spp
 // Cornell box and 111.6 ms for a 960x540 4-spp albedo pass over 200,000 triangles; one
-// active lane per warp 39.5 and 40.8 ms; this form 36.1 and 35.0 ms (passes on several streams overlap: 15.0 and 16.7 ms each).
+// active lane per warp 39.5 and 40.8 ms; this form 33.6 and 35.0 ms (passes on several streams
+// overlap: 16.6 and 16.7-23.8 ms each).
 #include <cuda_runtime.h>
 
 #include "pt_device.cuh"
