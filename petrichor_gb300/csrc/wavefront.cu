@@ -63,13 +63,19 @@ __device__ __forceinline__ int WarpAppend(int* counter, bool pred) {
 
 // ---------------------------------------------------------------- persistent tracer
 // Warp-persistent traversal with dynamic ray fetch: each warp pulls rays from a
-// queue counter and refills its idle lanes whenever half of the warp has
-// finished, so long rays do not hold a warp of finished lanes (the load
-// imbalance of incoherent secondary rays). A refill costs its 150 instructions and a trip to
-// the counter for however many lanes it fills: at 28, 24, 20, 16, 12 and 8 lanes left the
-// closest hits of the 1.0M-triangle 1080p frame took 17.80, 17.03, 16.22, 15.81, 15.66 and
-// 15.87 ms, its shadow rays 11.18, 11.00, 10.55, 10.28, 10.18 and 10.53 ms, and a closed
-// interior's frame 3.90 (24), 3.86 (20), 3.91 (16) and 3.94 ms (12). Bound by issue and by the warps' own
+// queue counter and refills its idle lanes once 20 of 32 have finished, so long rays do not
+// hold a warp of finished lanes (the load imbalance of incoherent secondary rays). A refill
+// costs its 150 instructions and a trip to the counter for however many lanes it fills.
+// Finished lanes keep their result until then and write all of them at once: a result's
+// reads and writes (for an area light, the whole of its contribution) stall the warp the same
+// for one lane as for twenty. With each lane's result written as its ray ended, a closed
+// interior's frame with an area light took 3.90 ms, the 1.0M-triangle 1080p frame 39.85, a
+// 2.2M-triangle 4K terrain frame 23.43 and a batch 12.65 ms; written at the refill 3.74, 39.59,
+// 23.30 and 12.54 ms, refilling at 16 lanes left. At 22, 19, 16, 14 and 12 lanes left they
+// take 3.75, 3.72, 3.73, 3.73 and 3.74; 40.79, 39.92, 39.41, 39.21 and 39.16; 23.90, 23.49, 23.23,
+// 23.11 and 23.05; 12.81, 12.63, 12.51, 12.48 and 12.47 ms; at 10 and 8 all are slower again, and
+// 4M incoherent rays with them (739 us at 12, 745 and 756).
+// Bound by issue and by the warps' own
 // latency: of 4M incoherent rays, 8 of 32 lanes were active per instruction, 70% of
 // issue slots busy and the L1 data pipe at 80%.
 constexpr unsigned kFullMask = 0xffffffffu;
@@ -378,7 +384,9 @@ __device__ void TraceQueue(Q& q, int n, int* fetch, int& err) {
     for (;;) {
         const unsigned idle = __ballot_sync(kFullMask, !active);
         const int nIdle = __popc(idle);
-        if (!exhausted && 32 - nIdle <= lim / 2) {
+        if (!exhausted && 32 - nIdle <= lim * 3 / 8) {
+            if (!active && idx >= 0) q.Finish(idx, r);
+            if (!active) idx = -1;
             const int take = min(nIdle, lim - (32 - nIdle));
             int first = 0;
             if (kFixedShare && lim <= 16) {
@@ -398,18 +406,15 @@ __device__ void TraceQueue(Q& q, int n, int* fetch, int& err) {
                 q.Load(idx, r);
                 r.Start();
                 stk.sp = 0;
-                if (r.nodes) {
-                    cur = 0;  // wide root
-                    active = true;
-                } else {
-                    q.Finish(idx, r);
-                }
+                cur = 0;  // wide root
+                active = r.nodes != nullptr;
             }
         }
         const unsigned busy = __ballot_sync(kFullMask, active);
         if (busy == 0) {
-            if (exhausted) break;
-            continue;
+            if (!exhausted) continue;
+            if (idx >= 0) q.Finish(idx, r);
+            break;
         }
         if (active) {
             bool done = false;
@@ -419,10 +424,7 @@ __device__ void TraceQueue(Q& q, int n, int* fetch, int& err) {
                 if (in == 0 || (__popc(in) <= kLeafLanes && in != busy)) break;
             }
             if (cur < 0 && cur != kDone) done = VisitLeaf<kAnyHit>(r, stk, cur, err);
-            if (done || cur == kDone) {
-                q.Finish(idx, r);
-                active = false;
-            }
+            if (done || cur == kDone) active = false;  // finished with the next refill
         }
     }
 }
