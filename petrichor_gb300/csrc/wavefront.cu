@@ -128,11 +128,12 @@ constexpr int kTraceBlock = 128;
 constexpr int kTraceWarps = kTraceBlock / 32;
 constexpr int kSmemStack = PT_SMEM_STACK;
 // A warp leaves the inner-node steps for its leaves once at most this many of its lanes
-// still hold an inner node (they wait): 2, 4, 8 and 12 measured 17.97, 17.77, 17.77 and
-// 17.79 ms for the closest hits of the 1.0M-triangle 1080p frame, against 18.90 with every
-// lane stepped to a leaf (0), and 748, 745 and 750 us for 4M incoherent rays (4, 8, 12)
-// against 787.
-constexpr int kLeafLanes = 4;
+// still hold an inner node (they wait). Stepping every lane to a leaf (0) took 18.90 ms for the
+// closest hits of the 1.0M-triangle 1080p frame where 4 took 17.77, and 787 us for 4M
+// incoherent rays where 4 took 748. With results written at the refill, 3, 4, 6 and 8 take
+// 15.47, 15.27, 15.10 and 15.15 ms (the frame 39.43, 39.18, 38.98 and 39.06), a 4K terrain
+// frame 23.20, 23.05, 22.94 and 22.98 ms, and the 4M rays 745, 740, 737 and 741 us.
+constexpr int kLeafLanes = 6;
 constexpr int kDone = INT_MIN;  // no further item (never a child code of a visited slot)
 
 struct TravStack {
