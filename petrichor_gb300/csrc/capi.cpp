@@ -501,6 +501,7 @@ int pt_context_destroy(pt_context* ctx) {
         Free(ctx, ctx->film);
         Free(ctx, ctx->stack);
         Free(ctx, ctx->status);
+        Free(ctx, ctx->rayCounter);
         Free(ctx, ctx->jobTable);
         Free(ctx, ctx->unitTable);
         Free(ctx, ctx->jobList);
@@ -1120,12 +1121,11 @@ int pt_trace_closest(pt_context* ctx, pt_scene_id scene, int32_t n, const float*
         return Fail(ctx, PT_ERR_INVALID_ARG, "bad ray buffers");
     int rc = SetDevice(ctx);
     if (rc != PT_OK) return rc;
-    const bool fresh = !ctx->status.ptr;
-    if ((rc = Alloc(ctx, ctx->status, 16)) != PT_OK) return rc;
-    // the first word is the status of tile renders, read back after every render
-    if (fresh) cudaMemset(ctx->status.ptr, 0, 16);
+    // a word of the queries' own, cleared on the launch's stream; the status buffer's first word
+    // is what tile renders report through
+    if ((rc = Alloc(ctx, ctx->rayCounter, 16)) != PT_OK) return rc;
     const cudaError_t e = LaunchTraceClosest(it->second->dev, n, rays, distMin, distMax, tri, dist,
-                                             (int*)ctx->status.ptr + 1,
+                                             (int*)ctx->rayCounter.ptr,
                                              stream ? (cudaStream_t)stream : ctx->stream);
     ctx->stats.kernel_launches++;
     return e == cudaSuccess ? PT_OK : CudaFail(ctx, e, "trace");

@@ -59,6 +59,7 @@ struct pt_context {
     int wbCapacity = 0;
     // scratch for host-film renders and replay stacks
     ptg::DeviceBuffer film, stack, status;
+    ptg::DeviceBuffer rayCounter;  // pt_trace_closest
     // wavefront job tables and per-job running sums
     ptg::DeviceBuffer jobTable, unitTable, jobList, accum;
     // launch configuration (pt_autotune / pt_set_tuning) and captured wave sequences
