@@ -213,7 +213,8 @@ WaveGraphCache* Graphs(pt_context* ctx) {
     return ctx->graphs;
 }
 
-int EnsureWaveBuffers(pt_context* ctx, int capacity) {
+// `stream`: the one whose kernels use the buffers next; new ones are cleared on it.
+int EnsureWaveBuffers(pt_context* ctx, int capacity, cudaStream_t stream) {
     if (ctx->wbCapacity >= capacity) return PT_OK;
     for (auto& b : ctx->wbBuffers) Free(ctx, b);
     ctx->wbBuffers.assign(1, DeviceBuffer{});
@@ -225,7 +226,8 @@ int EnsureWaveBuffers(pt_context* ctx, int capacity) {
     ctx->wb = CarveWaveBuffers(ctx->wbBuffers[0].ptr, capacity);
     ctx->wb.hostCount = hostCount;
     ctx->wb.bytes = bytes;
-    cudaMemsetAsync(ctx->wb.counts, 0, 16 * sizeof(int), ctx->stream);
+    const cudaError_t z = cudaMemsetAsync(ctx->wb.counts, 0, 16 * sizeof(int), stream);
+    if (z != cudaSuccess) return CudaFail(ctx, z, "wave counters");
     if (!ctx->wb.hostCount) {
         const cudaError_t e = cudaMallocHost(&ctx->wb.hostCount, sizeof(int) * 4);
         if (e != cudaSuccess) return CudaFail(ctx, e, "cudaMallocHost");
@@ -408,7 +410,7 @@ int RenderOnStream(pt_context* ctx, SceneGpu& sg, const pt_camera* cam, const pt
         }
     } else {
         const int cap = WaveCapacity(ctx, st);
-        int rc = EnsureWaveBuffers(ctx, cap);
+        int rc = EnsureWaveBuffers(ctx, cap, stream);
         if (rc != PT_OK) return rc;
         if ((rc = EnsureTables(ctx, 1, (size_t)st->width * st->height)) != PT_OK) return rc;
         DevJob job{};
@@ -985,7 +987,7 @@ int pt_render_profile(pt_context* ctx, pt_scene_id scene, const pt_camera* cam,
         return Fail(ctx, PT_ERR_UNSUPPORTED, "profiling covers the wavefront mode");
     if ((rc = SetDevice(ctx)) != PT_OK) return rc;
     const int cap = WaveCapacity(ctx, st);
-    if ((rc = EnsureWaveBuffers(ctx, cap)) != PT_OK) return rc;
+    if ((rc = EnsureWaveBuffers(ctx, cap, ctx->stream)) != PT_OK) return rc;
     if ((rc = EnsureTables(ctx, 1, (size_t)st->width * st->height)) != PT_OK) return rc;
     DeviceBuffer counters;
     if ((rc = Alloc(ctx, counters, 8 * sizeof(unsigned long long))) != PT_OK) return rc;
@@ -1052,7 +1054,7 @@ int pt_batch_render(pt_context* ctx, int32_t n, const pt_job* jobs, void* stream
     int rc = SetDevice(ctx);
     if (rc != PT_OK) return rc;
     const int cap = (int)std::max<int64_t>(std::min<int64_t>(paths, kMaxWavePaths), maxPx);
-    if ((rc = EnsureWaveBuffers(ctx, cap)) != PT_OK) return rc;
+    if ((rc = EnsureWaveBuffers(ctx, cap, stream ? (cudaStream_t)stream : ctx->stream)) != PT_OK) return rc;
     if ((rc = EnsureTables(ctx, n, pixels)) != PT_OK) return rc;
     size_t off = 0;
     for (int i = 0; i < n; i++) {
@@ -1145,7 +1147,7 @@ int pt_primary_hits(pt_context* ctx, pt_scene_id scene, const pt_camera* cam, co
     if ((int64_t)st->width * st->height * st->spp > cap)
         return Fail(ctx, PT_ERR_INVALID_ARG, "the camera rays do not fit in one wave");
     if ((rc = SetDevice(ctx)) != PT_OK) return rc;
-    if ((rc = EnsureWaveBuffers(ctx, cap)) != PT_OK) return rc;
+    if ((rc = EnsureWaveBuffers(ctx, cap, stream ? (cudaStream_t)stream : ctx->stream)) != PT_OK) return rc;
     if ((rc = EnsureTables(ctx, 1, (size_t)st->width * st->height)) != PT_OK) return rc;
     std::vector<DevJob> jobs(1);
     jobs[0].S = JobScene(*sg, st);

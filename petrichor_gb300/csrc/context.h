@@ -90,7 +90,7 @@ int CudaFail(pt_context* ctx, cudaError_t e, const char* what);
 int Alloc(pt_context* ctx, DeviceBuffer& b, size_t bytes);
 void Free(pt_context* ctx, DeviceBuffer& b);
 int SetDevice(pt_context* ctx);
-int EnsureWaveBuffers(pt_context* ctx, int capacity);
+int EnsureWaveBuffers(pt_context* ctx, int capacity, cudaStream_t stream);
 int CheckArgs(pt_context* ctx, pt_scene_id scene, const pt_camera* cam, const pt_settings* st,
               SceneGpu** out);
 DevCamera ToDev(const pt_camera* c);

@@ -1,5 +1,5 @@
-"""The host side of ray queries (csrc/capi.cpp pt_trace_closest) over a fake CUDA runtime
-(tests/cpp/fake_cuda.h): what a query enqueues, on which stream, and which words it uses."""
+"""The host side of device calls (csrc/capi.cpp) over a fake CUDA runtime
+(tests/cpp/fake_cuda.h): what a call enqueues, on which stream, and which words it uses."""
 import os
 import subprocess
 
@@ -43,3 +43,7 @@ def run_client(objs, source, exe, *args):
 
 def test_a_query_works_on_its_own_stream_alone(host_objects, tmp_path):
     assert run_client(host_objects, "ray_query.cpp", str(tmp_path / "ray_query")).startswith("ok")
+
+
+def test_a_render_clears_its_wave_buffers_on_its_own_stream(host_objects, tmp_path):
+    assert run_client(host_objects, "render_stream.cpp", str(tmp_path / "render_stream")).startswith("ok")
