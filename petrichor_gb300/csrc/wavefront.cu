@@ -22,6 +22,7 @@
 
 #include "pt_device.cuh"
 #include "pt_kernels.h"
+#include "query_share.h"
 #include "slab.h"
 
 namespace ptg {
@@ -349,12 +350,11 @@ __device__ __noinline__ void ResolveTie(const DevScene* S, V3 o, V3 d, float tmi
 // 427,180 paths and 4 bounces took 212 us unspread and 202, 202, 217 and 242 us with 4, 8, 16
 // and 28 warps per SM; a 512x288 4-spp frame of 20,000 triangles 869 us unspread, 650, 645,
 // 650 and 666 us.
-constexpr int kSpreadWarps = 6;
 __device__ __forceinline__ int LanesUsed(int n) {
     unsigned sms;
     asm("mov.u32 %0, %%nsmid;" : "=r"(sms));
     const int warps = (int)sms * kSpreadWarps;
-    return min(32, max(1, (n + warps - 1) / warps));
+    return min(32, (n - 1) / warps + 1);
 }
 
 // Q provides: void Load(int i, LaneRay&) (ray, range, and the scene: nodes = nullptr
@@ -362,17 +362,17 @@ __device__ __forceinline__ int LanesUsed(int n) {
 // will be loaded soon).
 // Must be called by every lane of the warp, in blocks of kTraceBlock threads.
 // kAnyHit: every ray Q loads is an any-hit ray.
-// kFixedShare: each warp takes its share of a short queue by its index instead of from the
-// counter. Two round trips to the counter fewer: 22.3 -> 21.4 us for 1000 rays, 37.5 -> 36.0
-// us for 4000; in the wave's trace kernels the extra code costs registers (an interior
-// frame 4.28 -> 4.44 ms), so only the ray queries use it.
+// kFixedShare, with share > 0: each warp takes `share` entries by its index instead of from
+// the counter (QueryShare: the shares cover the queue). Two round trips to the counter fewer:
+// 22.3 -> 21.4 us for 1000 rays, 37.5 -> 36.0 us for 4000; in the wave's trace kernels the
+// extra code costs registers (an interior frame 4.28 -> 4.44 ms), so only the ray queries use it.
 template <bool kAnyHit, bool kFixedShare = false, class Q>
-__device__ void TraceQueue(Q& q, int n, int* fetch, int& err) {
+__device__ void TraceQueue(Q& q, int n, int* fetch, int& err, int share = 0) {
     __shared__ int2 sEnt[!kAnyHit && kSmemStack > 0 ? kSmemStack * kTraceBlock : 1];
     __shared__ int sCode[kAnyHit && kSmemStack > 0 ? kSmemStack * kTraceBlock : 1];
     const int lane = threadIdx.x & 31;
     const unsigned lowerLanes = (1u << lane) - 1u;
-    const int lim = LanesUsed(n);
+    const int lim = kFixedShare && share > 0 ? share : LanesUsed(n);
     LaneRay r;
     int idx = -1;
     bool active = false;
@@ -389,18 +389,18 @@ __device__ void TraceQueue(Q& q, int n, int* fetch, int& err) {
             if (!active && idx >= 0) q.Finish(idx, r);
             if (!active) idx = -1;
             const int take = min(nIdle, lim - (32 - nIdle));
-            int first = 0;
-            if (kFixedShare && lim <= 16) {
+            unsigned first = 0;  // past n by the warps' last fetches: more than an int for the longest queues
+            if (kFixedShare && share > 0) {
                 first = (blockIdx.x * kTraceWarps + (threadIdx.x >> 5)) * lim;
                 exhausted = true;
             } else {
-                if (lane == 0) first = atomicAdd(fetch, take);
+                if (lane == 0) first = (unsigned)atomicAdd(fetch, take);
                 first = __shfl_sync(kFullMask, first, 0);
-                exhausted = first + take >= n;
+                exhausted = first + take >= (unsigned)n;
             }
             const int k = __popc(idle & lowerLanes);
-            if (!active && k < take && first + k < n) {
-                idx = first + k;
+            if (!active && k < take && first + k < (unsigned)n) {
+                idx = (int)(first + k);
                 // about one refill of every warp ahead; all warps together cover the queue
                 const int ahead = kTraceBlock / 2 * (int)gridDim.x;
                 if (idx < n - ahead) q.Prefetch(idx + ahead);
@@ -1261,11 +1261,11 @@ struct RayBatchQueue {
 
 __global__ void __launch_bounds__(128) TraceKernel(DevScene S, int n, const float* __restrict__ rays,
                                                    float tmin, float tmax, int* __restrict__ triOut,
-                                                   float* __restrict__ distOut, int* fetch) {
+                                                   float* __restrict__ distOut, int* fetch, int share) {
     RayBatchQueue q{&S, S.numWide > 0 ? S.wide : nullptr, S.tris, S.numWide, S.numTris, rays, tmin,
                     tmax, triOut, distOut};
     int err = 0;
-    TraceQueue<false, true>(q, n, fetch, err);
+    TraceQueue<false, true>(q, n, fetch, err, share);
 }
 
 // Profiling helpers: ray tallies and the reference traversal's work per ray.
@@ -1972,8 +1972,9 @@ cudaError_t LaunchTraceClosest(const DevScene& S, int n, const float* rays, floa
     if (n <= 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(fetchCounter, 0, sizeof(int), stream);
     if (e != cudaSuccess) return e;
-    TraceKernel<<<DefaultStageGrid(), 128, 0, stream>>>(S, n, rays, distMin, distMax, triOut, distOut,
-                                                        fetchCounter);
+    const int grid = DefaultStageGrid();
+    TraceKernel<<<grid, kTraceBlock, 0, stream>>>(S, n, rays, distMin, distMax, triOut, distOut, fetchCounter,
+                                                  QueryShare(n, SmCount(), grid * kTraceWarps));
     return cudaGetLastError();
 }
 
