@@ -287,7 +287,8 @@ int pt_serve_release(pt_context* ctx, uint64_t request_id);
 int pt_serve_stop(pt_context* ctx);
 
 /* Closest hits for n device rays (o.xyz, dir.xyz) within [dist_min, dist_max]:
- * original triangle index (or -1) and distance (or -1). Enqueued on `stream`. */
+ * original triangle index (or -1) and distance (or -1). Enqueued on `stream`; queries on
+ * several streams may run at the same time (of captured ones, up to 16 of a context). */
 int pt_trace_closest(pt_context* ctx, pt_scene_id scene, int32_t n, const float* rays_device,
                      float dist_min, float dist_max, int32_t* tri_device, float* dist_device,
                      void* stream);

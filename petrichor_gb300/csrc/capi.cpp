@@ -503,7 +503,9 @@ int pt_context_destroy(pt_context* ctx) {
         Free(ctx, ctx->film);
         Free(ctx, ctx->stack);
         Free(ctx, ctx->status);
-        Free(ctx, ctx->rayCounter);
+        Free(ctx, ctx->rayCounters.words);
+        for (cudaEvent_t ev : ctx->rayCounters.done)
+            if (ev) cudaEventDestroy(ev);
         Free(ctx, ctx->jobTable);
         Free(ctx, ctx->unitTable);
         Free(ctx, ctx->jobList);
@@ -1113,6 +1115,30 @@ int pt_render_replay_noalloc(pt_context* ctx, pt_scene_id scene, const pt_camera
     return PT_OK;
 }
 
+// A counter for a query about to be launched on `s`, and the event to record behind it (null:
+// `s` is being captured).
+static int TakeQueryCounter(pt_context* ctx, cudaStream_t s, int** counter, cudaEvent_t* done) {
+    QueryCounters& q = ctx->rayCounters;
+    const int rc = Alloc(ctx, q.words, 2 * QueryCounters::kTurns * sizeof(int));
+    if (rc != PT_OK) return rc;
+    int* words = (int*)q.words.ptr;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(s, &cs);
+    if (e != cudaSuccess) return CudaFail(ctx, e, "trace");
+    if (cs != cudaStreamCaptureStatusNone) {
+        *counter = words + QueryCounters::kTurns + q.nextCaptured;
+        q.nextCaptured = (q.nextCaptured + 1) % QueryCounters::kTurns;
+        return PT_OK;
+    }
+    cudaEvent_t& turn = q.done[q.next];
+    e = turn ? cudaStreamWaitEvent(s, turn, 0) : cudaEventCreateWithFlags(&turn, cudaEventDisableTiming);
+    if (e != cudaSuccess) return CudaFail(ctx, e, "trace");
+    *counter = words + q.next;
+    *done = turn;
+    q.next = (q.next + 1) % QueryCounters::kTurns;
+    return PT_OK;
+}
+
 int pt_trace_closest(pt_context* ctx, pt_scene_id scene, int32_t n, const float* rays,
                      float distMin, float distMax, int32_t* tri, float* dist, void* stream) {
     if (!ctx) return PT_ERR_INVALID_ARG;
@@ -1123,12 +1149,12 @@ int pt_trace_closest(pt_context* ctx, pt_scene_id scene, int32_t n, const float*
         return Fail(ctx, PT_ERR_INVALID_ARG, "bad ray buffers");
     int rc = SetDevice(ctx);
     if (rc != PT_OK) return rc;
-    // a word of the queries' own, cleared on the launch's stream; the status buffer's first word
-    // is what tile renders report through
-    if ((rc = Alloc(ctx, ctx->rayCounter, 16)) != PT_OK) return rc;
-    const cudaError_t e = LaunchTraceClosest(it->second->dev, n, rays, distMin, distMax, tri, dist,
-                                             (int*)ctx->rayCounter.ptr,
-                                             stream ? (cudaStream_t)stream : ctx->stream);
+    const cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
+    int* counter = nullptr;
+    cudaEvent_t done = nullptr;
+    if (TraceUsesCounter(n) && (rc = TakeQueryCounter(ctx, s, &counter, &done)) != PT_OK) return rc;
+    cudaError_t e = LaunchTraceClosest(it->second->dev, n, rays, distMin, distMax, tri, dist, counter, s);
+    if (e == cudaSuccess && done) e = cudaEventRecord(done, s);
     ctx->stats.kernel_launches++;
     return e == cudaSuccess ? PT_OK : CudaFail(ctx, e, "trace");
 }

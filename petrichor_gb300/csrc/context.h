@@ -31,6 +31,19 @@ struct SceneGpu {
     const float4* envAlias = nullptr;
 };
 
+// Fetch counters of long ray queries, one per query that may be running: queries of different
+// streams run at the same time, and one that shared a counter with another would skip the rays the
+// other took. A counter is used again behind an event recorded after the query that had
+// it. Events of a captured query exist only inside its graph, so captured queries take their
+// counters from a part of their own, in turn: up to kTurns of a context's captured queries may
+// run at the same time.
+struct QueryCounters {
+    static constexpr int kTurns = 16;
+    DeviceBuffer words;  // 2 kTurns: the others', then the captured ones'
+    cudaEvent_t done[kTurns] = {};
+    int next = 0, nextCaptured = 0;
+};
+
 class Server;  // server.cpp
 
 // Paths per wave: the whole image x spp when it fits, otherwise full sample blocks.
@@ -59,7 +72,7 @@ struct pt_context {
     int wbCapacity = 0;
     // scratch for host-film renders and replay stacks
     ptg::DeviceBuffer film, stack, status;
-    ptg::DeviceBuffer rayCounter;  // pt_trace_closest
+    ptg::QueryCounters rayCounters;  // pt_trace_closest
     // wavefront job tables and per-job running sums
     ptg::DeviceBuffer jobTable, unitTable, jobList, accum;
     // launch configuration (pt_autotune / pt_set_tuning) and captured wave sequences

@@ -181,7 +181,10 @@ cudaError_t RunPrimaryHits(const DevJob* jobs, const WaveUnit* units, const Wave
                            int* triOut, float* distOut, cudaStream_t stream, int* launches);
 
 // Closest-hit traversal of the throughput path for caller rays (o.xyz, d.xyz per ray).
-// fetchCounter: one device int of scratch for the persistent fetch.
+// fetchCounter: a device int for the persistent fetch, cleared here and the query's alone until
+// it has run; not used (may be null) by a short query (TraceUsesCounter false), whose warps
+// take their rays by index.
+bool TraceUsesCounter(int n);
 cudaError_t LaunchTraceClosest(const DevScene& S, int n, const float* rays, float distMin,
                                float distMax, int* triOut, float* distOut, int* fetchCounter,
                                cudaStream_t stream);

@@ -1966,15 +1966,20 @@ cudaError_t RunPrimaryHits(const DevJob* jobs, const WaveUnit* units, const Wave
     return cudaGetLastError();
 }
 
+static int TraceShare(int n) { return QueryShare(n, SmCount(), DefaultStageGrid() * kTraceWarps); }
+bool TraceUsesCounter(int n) { return n > 0 && TraceShare(n) == 0; }
+
 cudaError_t LaunchTraceClosest(const DevScene& S, int n, const float* rays, float distMin,
                                float distMax, int* triOut, float* distOut, int* fetchCounter,
                                cudaStream_t stream) {
     if (n <= 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(fetchCounter, 0, sizeof(int), stream);
-    if (e != cudaSuccess) return e;
-    const int grid = DefaultStageGrid();
-    TraceKernel<<<grid, kTraceBlock, 0, stream>>>(S, n, rays, distMin, distMax, triOut, distOut, fetchCounter,
-                                                  QueryShare(n, SmCount(), grid * kTraceWarps));
+    const int share = TraceShare(n);
+    if (share == 0) {
+        const cudaError_t e = cudaMemsetAsync(fetchCounter, 0, sizeof(int), stream);
+        if (e != cudaSuccess) return e;
+    }
+    TraceKernel<<<DefaultStageGrid(), kTraceBlock, 0, stream>>>(S, n, rays, distMin, distMax, triOut, distOut,
+                                                                fetchCounter, share);
     return cudaGetLastError();
 }
 
