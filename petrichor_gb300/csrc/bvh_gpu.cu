@@ -1110,13 +1110,16 @@ struct BuildArrays {
     Counters* cnt;
     int *ic, *index, *rank;
     OutNode* outNodes;
+    size_t scratch;  // where the arrays begin that only the build uses
     void Carve(Arena& ar, int T, int numVertices, int nodeCap, int activeCap, int segCap, int smallCap, int heapCap) {
         const size_t t = (size_t)T;
         dPos = ar.Get<float>(3 * (size_t)numVertices);
         dIdx = ar.Get<int32_t>(3 * t);
+        ids = ar.Get<int>(t);
+        outNodes = ar.Get<OutNode>(nodeCap);
+        scratch = ar.used;  // what follows is not kept
         cent = ar.Get<float>(3 * t);
         box = ar.Get<float>(6 * t);
-        ids = ar.Get<int>(t);
         key = ar.Get<float>(t);
         nodeOf = ar.Get<int>(t);
         seg = ar.Get<int>(t);
@@ -1150,7 +1153,6 @@ struct BuildArrays {
         ic = ar.Get<int>(nodeCap);
         index = ar.Get<int>(nodeCap);
         rank = ar.Get<int>(nodeCap);
-        outNodes = ar.Get<OutNode>(nodeCap);
     }
 };
 
@@ -1411,7 +1413,8 @@ cudaError_t BuildBinnedSahDevice(const float* positions, int numVertices, const 
     }
     out->height = numLevels - 1;
     if (keep) {
-        *keep = DeviceBvh{block.p, dPos, dIdx, reinterpret_cast<const BvhNodeOut*>(outNodes), ids};
+        *keep = DeviceBvh{block.p, dPos, dIdx, reinterpret_cast<const BvhNodeOut*>(outNodes), ids,
+                          static_cast<char*>(block.p) + arrays.scratch, ar.used - arrays.scratch};
         block.p = nullptr;
     }
     if (stats) {

@@ -60,6 +60,7 @@ int Alloc(pt_context* ctx, DeviceBuffer& b, size_t bytes) {
     if (bytes == 0) return PT_OK;
     const cudaError_t e = cudaMalloc(&b.ptr, bytes);
     if (e != cudaSuccess) {
+        cudaGetLastError();  // not the next launch's error
         b.ptr = nullptr;
         return Fail(ctx, PT_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
@@ -446,6 +447,109 @@ int FinishStats(pt_context* ctx, cudaStream_t stream) {
     return PT_OK;
 }
 
+namespace {
+// Device memory of one upload beside the scene's own buffers: one block that holds the sources
+// of the records, which is the build's where there was one (its arrays are sources, its free
+// part takes the others). Where memory is too short for the block beside the scene, an upload
+// goes on without it: each step's sources have allocations of their own, freed as soon as
+// the step has run, so that it needs at most one step's (39 bytes a triangle at half a vertex a
+// triangle, or part of an image) beside the scene. None of it counts in the budget.
+struct UploadScratch {
+    cudaStream_t stream;
+    DeviceBvh kept;
+    void* block = nullptr;
+    char* spare = nullptr;  // the block's free part
+    size_t spareBytes = 0, taken = 0;
+    std::vector<void*> own;
+    cudaError_t error = cudaSuccess;  // the first failure of this step
+
+    explicit UploadScratch(cudaStream_t s) : stream(s) {}
+    UploadScratch(const UploadScratch&) = delete;
+    ~UploadScratch() {
+        DropOwn();
+        DropBlock();
+    }
+    void DropOwn() {
+        for (void* p : own) cudaFree(p);  // waits for the device
+        own.clear();
+    }
+    void DropBlock() {
+        if (block) cudaFree(block);
+        block = nullptr;
+        kept = DeviceBvh{};
+        spareBytes = taken = 0;
+    }
+    // The build's block, or one of `bytes` where there was no build on the device.
+    void Keep() {
+        block = kept.block;
+        spare = kept.spare;
+        spareBytes = kept.spareBytes;
+    }
+    void Reserve(size_t bytes) {
+        if (cudaMalloc(&block, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            block = nullptr;
+            return;
+        }
+        spare = static_cast<char*>(block);
+        spareBytes = bytes;
+    }
+    static size_t Up(size_t bytes) { return (bytes + 255) & ~size_t(255); }
+    void* Spare(size_t bytes) {
+        if (Up(bytes) > spareBytes - taken) return nullptr;
+        void* p = spare + taken;
+        taken += Up(bytes);
+        return p;
+    }
+    void* Own(size_t bytes) {
+        void* p = nullptr;
+        const cudaError_t e = cudaMalloc(&p, bytes);
+        if (e != cudaSuccess) {
+            cudaGetLastError();  // not the next launch's error
+            if (error == cudaSuccess) error = e;
+            return nullptr;
+        }
+        own.push_back(p);
+        return p;
+    }
+    // A host array's device copy; null without an array or on a failure.
+    template <class T>
+    const T* Lift(const T* host, size_t n) {
+        if (!host || n == 0 || error != cudaSuccess) return nullptr;
+        void* p = Spare(n * sizeof(T));
+        if (!p) p = Own(n * sizeof(T));
+        if (p) error = cudaMemcpyAsync(p, host, n * sizeof(T), cudaMemcpyHostToDevice, stream);
+        return static_cast<const T*>(p);
+    }
+    // A buffer through which `n` items are copied up `*part` at a time: all of them or kMostPart
+    // bytes, less where memory is short (64 KB at least).
+    static constexpr size_t kMostPart = size_t(64) << 20;
+    void* TakePart(size_t n, size_t size, size_t* part) {
+        if (error != cudaSuccess) return nullptr;
+        size_t items = std::min(n, std::max<size_t>(1, kMostPart / size));
+        void* p = Spare(items * size);
+        while (!p) {
+            error = cudaSuccess;
+            p = Own(items * size);
+            if (p || items * size <= size_t(64) << 10) break;
+            items /= 2;
+        }
+        *part = items;
+        return p;
+    }
+    // Ends a step of enqueued work with its error: gives its own allocations back.
+    int StepDone(pt_context* ctx, cudaError_t e) {
+        DropOwn();
+        taken = 0;
+        if (e == cudaSuccess) e = error;
+        error = cudaSuccess;
+        if (e == cudaSuccess) return PT_OK;
+        return e == cudaErrorMemoryAllocation ? Fail(ctx, PT_ERR_OUT_OF_MEMORY, "scene upload: allocation failed")
+                                              : CudaFail(ctx, e, "scene upload");
+    }
+};
+}  // namespace
+
 }  // namespace ptg
 
 extern "C" {
@@ -559,21 +663,15 @@ int pt_scene_upload(pt_context* ctx, const pt_scene_desc* d, pt_scene_id* out) {
     const int T = (int)d->num_triangles;
     const auto t0 = std::chrono::steady_clock::now();
     BvhResult bvh;
-    DeviceBvh kept;  // the build's device arrays, from which the scene's records are formed
-    // device memory of this call alone; freed after the stream has run (cudaFree waits)
-    struct Temporary {
-        std::vector<void*> ptrs;
-        ~Temporary() {
-            for (void* p : ptrs) cudaFree(p);
-        }
-    } temporary;
+    UploadScratch scratch(ctx->stream);
+    const DeviceBvh& kept = scratch.kept;  // the build's device arrays, sources of the records
     if (ctx->bvhBuilder == PT_BVH_BUILDER_DEVICE) {
         std::string why;
         const cudaError_t be = BuildBinnedSahDevice(d->positions, (int)d->num_vertices, d->indices, T,
-                                                    ctx->stream, &bvh, &why, nullptr, &kept);
-        temporary.ptrs.push_back(kept.block);
+                                                    ctx->stream, &bvh, &why, nullptr, &scratch.kept);
         if (be != cudaSuccess)
             return Fail(ctx, be == cudaErrorMemoryAllocation ? PT_ERR_OUT_OF_MEMORY : PT_ERR_CUDA, why);
+        scratch.Keep();
     } else {
         bvh = BuildBinnedSah(d->positions, d->indices, T, 0);
     }
@@ -646,77 +744,105 @@ int pt_scene_upload(pt_context* ctx, const pt_scene_desc* d, pt_scene_id* out) {
     const int W = d->env_width, H = d->env_height;
     SceneGpu& s = *sg;
     DevScene& D = s.dev;
-    float4 *tree = nullptr, *tris = nullptr, *shade = nullptr, *env = nullptr, *texels = nullptr, *uvs = nullptr;
     // the sampler's outcomes are tabled for maps it has a closed form for (EnvSample)
     const bool envTabled = W > 0 && (W & (W - 1)) == 0 && (H & (H - 1)) == 0 && W <= (1 << 22) && H <= kEnvTableRows;
     float4 *envTable = nullptr, *envTableExact = nullptr;
-    const size_t envTableBytes = 2 * (size_t)H * 2 * sizeof(float4);
-    const size_t slot3 = 3 * sizeof(float4);
     const bool withUV = anyUV || anyTex;
-    if ((rc = SceneBuffer(ctx, s, wideOffset * sizeof(float4) + wideF.size() * sizeof(float), &tree)) != PT_OK ||
-        (rc = SceneBuffer(ctx, s, (size_t)T * slot3, &tris)) != PT_OK ||
-        (rc = SceneBuffer(ctx, s, (size_t)T * slot3, &shade)) != PT_OK ||
-        (rc = Upload(ctx, s, mats, &D.mats)) != PT_OK || (rc = Upload(ctx, s, lights, &D.lights)) != PT_OK ||
-        (rc = SceneBuffer(ctx, s, std::max<size_t>((size_t)W * H, 1) * sizeof(float4), &env)) != PT_OK ||
-        (envTabled && (rc = SceneBuffer(ctx, s, envTableBytes, &envTable)) != PT_OK) ||
-        (envTabled && (rc = SceneBuffer(ctx, s, envTableBytes, &envTableExact)) != PT_OK) ||
-        (anyTex && (rc = SceneBuffer(ctx, s, std::max<size_t>(numTexels, 1) * sizeof(float4), &texels)) != PT_OK) ||
-        (anyTex && (rc = Upload(ctx, s, texInfo, &D.texInfo)) != PT_OK) ||
-        (withUV && (rc = SceneBuffer(ctx, s, (size_t)std::max(T, 1) * slot3, &uvs)) != PT_OK)) {
-        for (auto& b : s.buffers) Free(ctx, b);
-        return rc;
-    }
-    D.nodes = tree;
-    D.tris = tris;
-    D.shade = shade;
-    D.env = env;
-    D.texels = texels;
-    D.uvs = uvs;
-    // the caller's arrays on the device, for the kernels that form the records
-    cudaError_t e = cudaSuccess;
-    auto lift = [&](const void* host, size_t bytes) -> void* {
-        void* p = nullptr;
-        if (!host || bytes == 0 || e != cudaSuccess) return nullptr;
-        e = cudaMalloc(&p, bytes);
-        if (e != cudaSuccess) return nullptr;
-        temporary.ptrs.push_back(p);
-        e = cudaMemcpyAsync(p, host, bytes, cudaMemcpyHostToDevice, ctx->stream);
-        return p;
+    const size_t V = d->num_vertices, T1 = (size_t)T;
+    size_t largest = (size_t)W * H;  // texels of the largest image
+    for (uint32_t t = 0; anyTex && t < d->num_textures; t++)
+        largest = std::max(largest, (size_t)d->textures[t].width * d->textures[t].height);
+    // the scene's buffers and what is formed in them
+    auto form = [&]() -> int {
+        float4 *tree = nullptr, *tris = nullptr, *shade = nullptr, *env = nullptr, *texels = nullptr, *uvs = nullptr;
+        const size_t envTableBytes = 2 * (size_t)H * 2 * sizeof(float4);
+        const size_t slot3 = 3 * sizeof(float4);
+        int rc;
+        cudaError_t e = cudaSuccess;
+        if ((rc = Upload(ctx, s, mats, &D.mats)) != PT_OK || (rc = Upload(ctx, s, lights, &D.lights)) != PT_OK ||
+            (anyTex && (rc = Upload(ctx, s, texInfo, &D.texInfo)) != PT_OK) ||
+            (rc = SceneBuffer(ctx, s, wideOffset * sizeof(float4) + wideF.size() * sizeof(float), &tree)) != PT_OK ||
+            (rc = SceneBuffer(ctx, s, T1 * slot3, &tris)) != PT_OK)
+            return rc;
+        if (!wideF.empty())
+            e = cudaMemcpyAsync(tree + wideOffset, wideF.data(), wideF.size() * sizeof(float), cudaMemcpyHostToDevice,
+                                ctx->stream);
+        const BvhNodeOut* nodes = kept.nodes;
+        size_t part = bvh.nodes.size();
+        if (!kept.block) nodes = (const BvhNodeOut*)scratch.TakePart(bvh.nodes.size(), sizeof(BvhNodeOut), &part);
+        for (size_t k = 0; k < bvh.nodes.size() && e == cudaSuccess && nodes; k += part) {
+            const size_t n = std::min(part, bvh.nodes.size() - k);
+            if (!kept.block)
+                e = cudaMemcpyAsync((void*)nodes, bvh.nodes.data() + k, n * sizeof(BvhNodeOut), cudaMemcpyHostToDevice,
+                                    ctx->stream);
+            if (e == cudaSuccess)
+                e = FormNodeRecords(nodes, (int)k, (int)n, tree, (int)wideOffset, wideEps, tris, ctx->stream);
+        }
+        if ((rc = scratch.StepDone(ctx, e)) != PT_OK) return rc;
+        if ((rc = SceneBuffer(ctx, s, T1 * slot3, &shade)) != PT_OK ||
+            (withUV && (rc = SceneBuffer(ctx, s, std::max<size_t>(T1, 1) * slot3, &uvs)) != PT_OK))
+            return rc;
+        if (uvs) e = cudaMemsetAsync(uvs, 0, slot3, ctx->stream);
+        if (T > 0 && e == cudaSuccess) {
+            SceneArrays in{};
+            in.positions = kept.block ? kept.positions : scratch.Lift(d->positions, 3 * V);
+            in.indices = kept.block ? kept.indices : scratch.Lift(d->indices, 3 * T1);
+            in.primIds = kept.block ? kept.primIds : scratch.Lift(bvh.primIds.data(), T1);
+            in.normals = scratch.Lift(d->normals, 3 * V);
+            in.uvs = withUV ? scratch.Lift(d->uvs, 3 * V) : nullptr;
+            in.material = scratch.Lift(d->tri_material, T1);
+            in.shading = scratch.Lift(d->tri_shading, T1);
+            in.numTris = T;
+            if (scratch.error == cudaSuccess) e = FormSlotRecords(in, tris, shade, uvs, ctx->stream);
+        }
+        if ((rc = scratch.StepDone(ctx, e)) != PT_OK) return rc;
+        if ((rc = SceneBuffer(ctx, s, std::max<size_t>((size_t)W * H, 1) * sizeof(float4), &env)) != PT_OK ||
+            (envTabled && (rc = SceneBuffer(ctx, s, envTableBytes, &envTable)) != PT_OK) ||
+            (envTabled && (rc = SceneBuffer(ctx, s, envTableBytes, &envTableExact)) != PT_OK) ||
+            (anyTex && (rc = SceneBuffer(ctx, s, std::max<size_t>(numTexels, 1) * sizeof(float4), &texels)) != PT_OK))
+            return rc;
+        // the sky and the maps, in parts through one buffer
+        float* rgb = largest > 0 ? (float*)scratch.TakePart(largest, 3 * sizeof(float), &part) : nullptr;
+        auto pad = [&](const float* host, size_t n, float4* out) {
+            for (size_t k = 0; k < n && e == cudaSuccess && rgb; k += part) {
+                const size_t m = std::min(part, n - k);
+                e = cudaMemcpyAsync(rgb, host + 3 * k, 3 * sizeof(float) * m, cudaMemcpyHostToDevice, ctx->stream);
+                if (e == cudaSuccess) e = PadTexels(rgb, m, out + k, ctx->stream);
+            }
+        };
+        if (W > 0) pad(d->env_rgb, (size_t)W * H, env);
+        else e = cudaMemsetAsync(env, 0, sizeof(float4), ctx->stream);
+        for (uint32_t t = 0; anyTex && t < d->num_textures; t++)
+            pad(d->textures[t].rgb, (size_t)d->textures[t].width * d->textures[t].height, texels + texInfo[t].x);
+        if ((rc = scratch.StepDone(ctx, e)) != PT_OK) return rc;
+        D.nodes = tree;
+        D.tris = tris;
+        D.shade = shade;
+        D.env = env;
+        D.texels = texels;
+        D.uvs = uvs;
+        return PT_OK;
     };
-    const size_t V3 = 3 * sizeof(float) * (size_t)d->num_vertices, T1 = (size_t)T;
-    SceneArrays in{};
-    in.positions = kept.block ? kept.positions : (const float*)lift(d->positions, V3);
-    in.indices = kept.block ? kept.indices : (const int32_t*)lift(d->indices, 3 * sizeof(int32_t) * T1);
-    in.nodes = kept.block ? kept.nodes : (const BvhNodeOut*)lift(bvh.nodes.data(), bvh.nodes.size() * sizeof(BvhNodeOut));
-    in.primIds = kept.block ? kept.primIds : (const int32_t*)lift(bvh.primIds.data(), sizeof(int32_t) * T1);
-    in.normals = (const float*)lift(T > 0 ? d->normals : nullptr, V3);
-    in.uvs = (const float*)lift(T > 0 && withUV ? d->uvs : nullptr, V3);
-    in.material = (const int32_t*)lift(d->tri_material, sizeof(int32_t) * T1);
-    in.shading = (const uint8_t*)lift(d->tri_shading, T1);
-    in.numNodes = (int)bvh.nodes.size();
-    in.numTris = T;
-    if (e == cudaSuccess && !wideF.empty())
-        e = cudaMemcpyAsync(tree + wideOffset, wideF.data(), wideF.size() * sizeof(float), cudaMemcpyHostToDevice,
-                            ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(env, 0, sizeof(float4), ctx->stream);
-    if (e == cudaSuccess && uvs) e = cudaMemsetAsync(uvs, 0, slot3, ctx->stream);
-    if (e == cudaSuccess) e = FormSceneRecords(in, tree, (int)wideOffset, wideEps, tris, shade, uvs, ctx->stream);
-    if (e == cudaSuccess && W > 0) {
-        const float* rgb = (const float*)lift(d->env_rgb, 3 * sizeof(float) * (size_t)W * H);
-        if (e == cudaSuccess) e = PadTexels(rgb, (size_t)W * H, env, ctx->stream);
+    if (!scratch.block) {
+        auto up = UploadScratch::Up;
+        const size_t perVertex = up(12 * V) * (1 + (d->normals != nullptr) + (withUV && d->uvs != nullptr));
+        const size_t slots = T > 0 ? perVertex + up(12 * T1) + 2 * up(4 * T1) + up(T1) : 0;
+        const size_t parts = std::max(bvh.nodes.size() * sizeof(BvhNodeOut), 3 * sizeof(float) * largest);
+        scratch.Reserve(std::max(slots, up(std::min(parts, UploadScratch::kMostPart))));
     }
-    for (uint32_t t = 0; anyTex && t < d->num_textures && e == cudaSuccess; t++) {
-        const pt_texture& X = d->textures[t];
-        const size_t n = (size_t)X.width * X.height;
-        const float* rgb = (const float*)lift(X.rgb, 3 * sizeof(float) * n);
-        if (e == cudaSuccess) e = PadTexels(rgb, n, texels + texInfo[t].x, ctx->stream);
+    rc = form();
+    if (rc == PT_ERR_OUT_OF_MEMORY && scratch.block) {
+        // once more without the block, the sources copied up again a step at a time
+        for (auto& b : s.buffers) Free(ctx, b);
+        s.buffers.clear();
+        scratch.DropBlock();
+        rc = form();
+        if (rc == PT_OK) ctx->lastError.clear();
     }
-    if (e != cudaSuccess) {
-        cudaGetLastError();  // a failed allocation's error is not the next launch's
+    if (rc != PT_OK) {
         cudaStreamSynchronize(ctx->stream);
         for (auto& b : s.buffers) Free(ctx, b);
-        return e == cudaErrorMemoryAllocation ? Fail(ctx, PT_ERR_OUT_OF_MEMORY, "scene upload: allocation failed")
-                                              : CudaFail(ctx, e, "scene upload");
+        return rc;
     }
     D.wide = D.nodes + wideOffset;
     D.numNodes = T > 0 ? (int)bvh.nodes.size() : 0;
@@ -733,6 +859,7 @@ int pt_scene_upload(pt_context* ctx, const pt_scene_desc* d, pt_scene_id* out) {
     for (int a = 0; a < 3; a++) D.envBase[a] = d->env_base_color[a];
     D.envRot = d->env_z_rotation;
     D.lightPdfArea = 1.0f / sumArea;
+    cudaError_t e = cudaSuccess;
     if (envTabled) {
         e = FillEnvTable(D, envTable, ctx->stream);
         if (e == cudaSuccess) e = FillEnvTableExact(D, envTableExact, ctx->stream);

@@ -21,13 +21,15 @@ __device__ __forceinline__ void MarkBox(float4* tris, int slot, int node, int wi
     w[3] = eps;
 }
 
-__global__ void __launch_bounds__(kThreads) NodeRecords(SceneArrays in, float4* __restrict__ nodes, int wideOffset,
-                                                        float wideEps, float4* __restrict__ tris) {
-    const int i = blockIdx.x * kThreads + threadIdx.x;
+__global__ void __launch_bounds__(kThreads) NodeRecords(const BvhNodeOut* __restrict__ in, int first, int count,
+                                                        float4* __restrict__ nodes, int wideOffset, float wideEps,
+                                                        float4* __restrict__ tris) {
+    const int at = blockIdx.x * kThreads + threadIdx.x;
+    const int i = first + at;
     const int lane = threadIdx.x & 31;
     int begin = 0, end = 0;
-    if (i < in.numNodes) {
-        const BvhNodeOut n = in.nodes[i];
+    if (at < count) {
+        const BvhNodeOut n = in[at];
         nodes[2 * (size_t)i] = make_float4(n.lo[0], n.lo[1], n.lo[2], n.hi[0]);
         nodes[2 * (size_t)i + 1] = make_float4(n.hi[1], n.hi[2], __int_as_float(n.leaf ? n.begin : n.child[0]),
                                                __int_as_float(n.leaf ? n.end - n.begin : -1));
@@ -84,10 +86,14 @@ unsigned Blocks(size_t n) { return (unsigned)((n + kThreads - 1) / kThreads); }
 
 }  // namespace
 
-cudaError_t FormSceneRecords(const SceneArrays& in, float4* nodes, int wideOffset, float wideEps, float4* tris,
-                             float4* shade, float4* uvsOut, cudaStream_t stream) {
-    if (in.numNodes > 0)
-        NodeRecords<<<Blocks(in.numNodes), kThreads, 0, stream>>>(in, nodes, wideOffset, wideEps, tris);
+cudaError_t FormNodeRecords(const BvhNodeOut* in, int first, int count, float4* nodes, int wideOffset, float wideEps,
+                            float4* tris, cudaStream_t stream) {
+    if (count > 0)
+        NodeRecords<<<Blocks(count), kThreads, 0, stream>>>(in, first, count, nodes, wideOffset, wideEps, tris);
+    return cudaGetLastError();
+}
+
+cudaError_t FormSlotRecords(const SceneArrays& in, float4* tris, float4* shade, float4* uvsOut, cudaStream_t stream) {
     if (in.numTris > 0) SlotRecords<<<Blocks(in.numTris), kThreads, 0, stream>>>(in, tris, shade, uvsOut);
     return cudaGetLastError();
 }

@@ -24,6 +24,7 @@ struct Op {
 inline std::vector<Op> ops;
 inline std::map<void*, size_t> blocks;
 inline size_t inUse = 0, peak = 0, limit = 0;  // limit 0: none
+inline cudaError_t lastError = cudaSuccess;
 inline std::set<cudaStream_t> capturing;
 inline uintptr_t handles = 0x1000;
 
@@ -37,12 +38,15 @@ T Handle() {
 extern "C" {
 cudaError_t cudaGetDeviceCount(int* n) { return *n = 1, cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+    const cudaError_t e = fake::lastError;
+    return fake::lastError = cudaSuccess, e;
+}
 const char* cudaGetErrorString(cudaError_t e) { return e == cudaErrorMemoryAllocation ? "out of memory" : "error"; }
 cudaError_t cudaMalloc(void** p, size_t n) {
     *p = nullptr;
-    if (fake::limit && fake::inUse + n > fake::limit) return cudaErrorMemoryAllocation;
-    *p = std::malloc(n);
+    if (fake::limit && fake::inUse + n > fake::limit) return fake::lastError = cudaErrorMemoryAllocation;
+    *p = std::memset(std::malloc(n), 0xA5, n);
     fake::blocks[*p] = n;
     fake::inUse += n;
     if (fake::inUse > fake::peak) fake::peak = fake::inUse;

@@ -47,3 +47,8 @@ def test_a_query_works_on_its_own_stream_alone(host_objects, tmp_path):
 
 def test_a_render_clears_its_wave_buffers_on_its_own_stream(host_objects, tmp_path):
     assert run_client(host_objects, "render_stream.cpp", str(tmp_path / "render_stream")).startswith("ok")
+
+
+def test_an_upload_needs_no_more_than_the_build_or_the_scene(host_objects, tmp_path):
+    """Device memory of an upload: the larger of the build and the scene, and part of an image."""
+    assert run_client(host_objects, "upload_peak.cpp", str(tmp_path / "upload_peak")).startswith("ok")
