@@ -349,7 +349,8 @@ __device__ __noinline__ void ResolveTie(const DevScene* S, V3 o, V3 d, float tmi
 // busy, more warps with fewer lanes only issue more instructions: a Cornell frame of
 // 427,180 paths and 4 bounces took 212 us unspread and 202, 202, 217 and 242 us with 4, 8, 16
 // and 28 warps per SM; a 512x288 4-spp frame of 20,000 triangles 869 us unspread, 650, 645,
-// 650 and 666 us.
+// 650 and 666 us. (Ray queries have a spread of their own, query_share.h.)
+constexpr int kSpreadWarps = 6;
 __device__ __forceinline__ int LanesUsed(int n) {
     unsigned sms;
     asm("mov.u32 %0, %%nsmid;" : "=r"(sms));
@@ -363,8 +364,8 @@ __device__ __forceinline__ int LanesUsed(int n) {
 // Must be called by every lane of the warp, in blocks of kTraceBlock threads.
 // kAnyHit: every ray Q loads is an any-hit ray.
 // kFixedShare, with share > 0: each warp takes `share` entries by its index instead of from
-// the counter (QueryShare: the shares cover the queue). Two round trips to the counter fewer:
-// 22.3 -> 21.4 us for 1000 rays, 37.5 -> 36.0 us for 4000; in the wave's trace kernels the
+// the counter (QueryShare: the shares cover the queue). Two round trips to the counter fewer, and
+// its clear: 22.3 -> 16.9 us for 1000 rays at the same spread; in the wave's trace kernels the
 // extra code costs registers (an interior frame 4.28 -> 4.44 ms), so only the ray queries use it.
 template <bool kAnyHit, bool kFixedShare = false, class Q>
 __device__ void TraceQueue(Q& q, int n, int* fetch, int& err, int share = 0) {

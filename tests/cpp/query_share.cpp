@@ -20,9 +20,9 @@ int main() {
             }
     for (int n : {INT_MAX, INT_MAX - 1, INT_MAX - 911, 1 << 30})
         if (ptg::QueryShare(n, 152, 4864) != 0) return std::printf("%d rays are not short\n", n), 1;
-    // the sizes at which the spread ends on 152 SMs
-    if (ptg::QueryShare(912, 152, 4864) != 1 || ptg::QueryShare(913, 152, 4864) != 2 ||
-        ptg::QueryShare(16 * 912, 152, 4864) != 16 || ptg::QueryShare(16 * 912 + 1, 152, 4864) != 0)
+    // on 152 SMs with 8 blocks of 4 warps each: 4256 warps take up to 31 rays
+    if (ptg::QueryShare(4256, 152, 4864) != 1 || ptg::QueryShare(4257, 152, 4864) != 2 ||
+        ptg::QueryShare(31 * 4256, 152, 4864) != 31 || ptg::QueryShare(31 * 4256 + 1, 152, 4864) != 0)
         return std::printf("shares on 152 SMs differ\n"), 1;
     std::printf("ok %ld\n", queries);
     return 0;

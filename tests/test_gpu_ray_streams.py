@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-@pytest.mark.parametrize("n", [700, 16 * 6 * 152 + 1, 200_000])
+@pytest.mark.parametrize("n", [700, 31 * 28 * 152, 31 * 28 * 152 + 1, 200_000])
 def test_concurrent_queries(n):
     sc = synth.spheres_grids(seed=4, tri_budget=20_000, env_width=16, env_height=8)
     lo, hi = torch.tensor(sc.positions.min(0), device="cuda"), torch.tensor(sc.positions.max(0), device="cuda")
@@ -36,7 +36,7 @@ def test_concurrent_queries(n):
 
 def test_captured_query_replays():
     """A captured query, replayed beside direct ones on another stream."""
-    n = 100_000
+    n = 150_000
     sc = synth.spheres_grids(seed=4, tri_budget=20_000, env_width=16, env_height=8)
     rays = torch.randn(n, 6, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
     tri = torch.full((3, n), -7, dtype=torch.int32, device="cuda")
