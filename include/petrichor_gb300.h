@@ -379,7 +379,9 @@ typedef struct pt_tuning {
   int32_t band_rows;     /* rows per pixel band of the path order (0: 8) */
   int32_t use_graphs;    /* 1: replay each wave's stage sequence from a captured CUDA graph */
   int32_t sort_rays;     /* 1: reorder each bounce's rays by direction and origin cell */
-  int32_t tail_bounce;   /* > 0: from this bounce on, one launch finishes every path (0: off) */
+  int32_t tail_bounce;   /* > 0: from this bounce on, one launch finishes every path; -1: never,
+                            every wave runs all its stages; 0: where few paths are left, which
+                            a small wave's are from the start */
   int32_t primary_traversal; /* first-bounce rays of a pinhole PathTracing job: 0 rasterised
                                 when the unit has at least 16 rays per triangle, else traced;
                                 1 always traced through the BVH; 2 rasterised whenever the

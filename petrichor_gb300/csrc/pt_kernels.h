@@ -136,7 +136,8 @@ struct WaveTuning {
     int band = 0;         // rows per pixel band of the path order (0: 8)
     int graphs = 1;       // replay each wave's stage sequence from a captured CUDA graph
     int sortRays = 0;     // reorder each bounce's rays by direction and origin cell before tracing
-    int tailBounce = 0;   // > 0: from this bounce on, one launch finishes every path (TailKernel)
+    int tailBounce = 0;   // > 0: from this bounce on, one launch finishes every path (TailKernel);
+                          // 0: where few paths are left; -1: never
     // first bounce: 0 rasterised for units with enough rays per triangle, else traced;
     // 1 always traced through the BVH; 2 rasterised wherever the camera allows it
     int primaryTraversal = 0;

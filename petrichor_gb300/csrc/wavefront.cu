@@ -1667,11 +1667,12 @@ struct WaveGraphKey {
     const void* jobs;
     const void* units;
     const void* buffers;
-    int capacity, iters, integrator, grid, sort, accum, tail, raster, envOnly;
+    int capacity, iters, integrator, grid, sort, accum, tail, raster, envOnly, mayTail, shadeGrid;
     bool operator==(const WaveGraphKey& o) const {
         return jobs == o.jobs && units == o.units && buffers == o.buffers && capacity == o.capacity &&
                iters == o.iters && integrator == o.integrator && grid == o.grid && sort == o.sort &&
-               accum == o.accum && tail == o.tail && raster == o.raster && envOnly == o.envOnly;
+               accum == o.accum && tail == o.tail && raster == o.raster && envOnly == o.envOnly &&
+               mayTail == o.mayTail && shadeGrid == o.shadeGrid;
     }
 };
 struct WaveGraph {
@@ -1780,7 +1781,8 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
     d.band = tune.band > 0 ? tune.band : 8;
     // the first bounce rasterised where the wave allows it (raster_primary.cuh)
     const bool sort = tune.sortRays != 0;
-    const bool whole = !prof && !sort && shape.nPaths <= kTailWavePaths;
+    const bool mayTail = !prof && !sort && tune.tailBounce >= 0;
+    const bool whole = mayTail && tune.tailBounce == 0 && shape.nPaths <= kTailWavePaths;
     const bool raster = !whole && shape.raster > 0 && tune.primaryTraversal != 1 && tune.sortRays == 0 &&
                         shape.iters >= 0;
     d.rasterFrom = raster ? shape.rasterFrom : shape.nPaths;
@@ -1792,7 +1794,7 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
     int nl = 0;
     // the last bounces in one launch (fixed-depth waves; profiled renders keep every stage)
     const int tailFrom = whole ? 0
-                         : (!prof && !sort && tune.tailBounce > 0 && shape.iters > tune.tailBounce)
+                         : (mayTail && tune.tailBounce > 0 && shape.iters > tune.tailBounce)
                            ? tune.tailBounce : -1;
     // shadow stages beside the next extend, on the owner's side stream (not when profiling,
     // whose stage timers need one stream)
@@ -1801,13 +1803,14 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
     const bool envOnly = !shape.areaLights;
     const int visit = RasterVisitClass(shape);
     const WaveGraphKey key{jobs, units, wb.ray[0], wb.capacity, shape.iters, shape.integrator, grid,
-                           sort ? 1 : 0, accumulate ? 1 : 0, tailFrom, raster ? 1 + visit : 0, envOnly ? 1 : 0};
+                           sort ? 1 : 0, accumulate ? 1 : 0, tailFrom, raster ? 1 + visit : 0, envOnly ? 1 : 0,
+                           mayTail ? 1 : 0, sgrid};
     if (shape.iters >= 0 || whole) {
         const int iters = shape.iters >= 0 ? shape.iters : kMaxReplayBounces;
         auto record = [&](int* n) {
             RaygenKernel<<<grid, block, 0, stream>>>(jobs, units, wb, 0, raster ? 1 : 0, whole ? 1 : 0);
             LaunchBounces(jobs, units, wb, shape.integrator, grid, sgrid, 0, iters, stream, prof, n, sort,
-                          ov, envOnly, true, tailFrom, raster, !sort, visit);
+                          ov, envOnly, true, tailFrom, raster, mayTail, visit);
             if (accumulate) AccumulateKernel<<<grid, block, 0, stream>>>(jobs, units, wb);
             *n += accumulate ? 2 : 1;
         };
@@ -1818,7 +1821,7 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
             RaygenKernel<<<grid, block, 0, stream>>>(jobs, units, wb, 0, raster ? 1 : 0, whole ? 1 : 0);
             if (ev) ev->End(0, stream);
             LaunchBounces(jobs, units, wb, shape.integrator, grid, sgrid, 0, iters, stream, prof, &nl, sort,
-                          ov, envOnly, true, tailFrom, raster, !sort && !prof, visit);
+                          ov, envOnly, true, tailFrom, raster, mayTail, visit);
             if (accumulate) {
                 if (ev) ev->Begin(4, stream);
                 AccumulateKernel<<<grid, block, 0, stream>>>(jobs, units, wb);
@@ -1838,7 +1841,7 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
                 e = cudaMemcpyAsync(wb.hostCount, wb.counts, sizeof(int), cudaMemcpyDeviceToHost, stream);
                 if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
                 if (e != cudaSuccess || *wb.hostCount == 0 || it >= kMaxReplayBounces) break;
-                if (!prof && !sort && *wb.hostCount <= kTailPaths) {
+                if (mayTail && *wb.hostCount <= kTailPaths) {
                     LaunchTail(jobs, wb, shape.integrator, 0, kMaxReplayBounces - it, INT_MAX, stream);
                     nl++;
                     break;
