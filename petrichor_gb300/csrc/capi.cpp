@@ -355,6 +355,12 @@ DevScene JobScene(const SceneGpu& s, const pt_settings* st) {
     return S;
 }
 
+int CameraInside(const SceneGpu& s, const pt_camera* c) {
+    for (int a = 0; a < 3; a++)
+        if (!(s.lo[a] <= c->pos[a] && c->pos[a] <= s.hi[a])) return 0;
+    return s.dev.numTris > 0 ? 1 : 0;
+}
+
 DevCamera ToDev(const pt_camera* c) {
     DevCamera d{};
     for (int a = 0; a < 3; a++) {
@@ -418,6 +424,7 @@ int RenderOnStream(pt_context* ctx, SceneGpu& sg, const pt_camera* cam, const pt
         job.S = JobScene(sg, st);
         job.C = C;
         job.st = S;
+        job.inside = CameraInside(sg, cam);
         job.accum = (float4*)ctx->accum.ptr;
         job.film = dFilm;
         e = RenderJobs({job}, Tables(ctx), ctx->wb, cap, stream, &launches, nullptr, ctx->tuning,
@@ -876,6 +883,10 @@ int pt_scene_upload(pt_context* ctx, const pt_scene_desc* d, pt_scene_id* out) {
         return Fail(ctx, PT_ERR_UNSUPPORTED, "BVH height " + std::to_string(bvh.height) +
                                                  " exceeds the traversal stack");
     }
+    for (int a = 0; a < 3; a++) {
+        s.lo[a] = bvh.nodes[0].lo[a];
+        s.hi[a] = bvh.nodes[0].hi[a];
+    }
     s.info.num_triangles = T;
     s.info.num_nodes = (uint32_t)bvh.nodes.size();
     s.info.tree_height = bvh.height;
@@ -1173,6 +1184,7 @@ int pt_batch_render(pt_context* ctx, int32_t n, const pt_job* jobs, void* stream
         if (!jobs[i].film_device) return Fail(ctx, PT_ERR_INVALID_ARG, "job film is NULL");
         dj[i].S = JobScene(*sg, &jobs[i].settings);
         dj[i].C = ToDev(&jobs[i].camera);
+        dj[i].inside = CameraInside(*sg, &jobs[i].camera);
         dj[i].st = ToDev(&jobs[i].settings);
         dj[i].film = jobs[i].film_device;
         const int P = jobs[i].settings.width * jobs[i].settings.height;

@@ -25,6 +25,7 @@ struct SceneGpu {
     DevScene dev{};
     std::vector<DeviceBuffer> buffers;
     pt_scene_info info{};
+    float lo[3] = {}, hi[3] = {};  // bounds of the triangles
     std::atomic<int> refs{0};  // serving requests that use the scene
     // alias table of the optional environment sampler, built at the first render that
     // asks for it (owned by buffers)
@@ -108,6 +109,8 @@ int CheckArgs(pt_context* ctx, pt_scene_id scene, const pt_camera* cam, const pt
               SceneGpu** out);
 DevCamera ToDev(const pt_camera* c);
 DevSettings ToDev(const pt_settings* s);
+// Whether the camera lies within the bounds of the scene's triangles.
+int CameraInside(const SceneGpu& s, const pt_camera* c);
 // The scene as one job sees it: the environment alias table attached when the
 // settings ask for it (CheckArgs has built it).
 DevScene JobScene(const SceneGpu& s, const pt_settings* st);

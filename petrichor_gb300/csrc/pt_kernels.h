@@ -51,7 +51,8 @@ struct DevJob {
     DevSettings st;
     float4* accum;  // width*height running sums {rgb, 0}; zeroed before the job's first wave
     float* film;    // width*height*3 output, written by FinalizeJobs
-    int32_t pad[4];
+    int32_t inside;  // the camera lies within the scene's bounds (CameraInside)
+    int32_t pad[3];
 };
 
 // One job's samples [s0, s0 + sw) over all its pixels: paths
@@ -125,11 +126,14 @@ struct WaveShape {
     int nUnits = 0, nPaths = 0, nPixelUnits = 0;
     int iters = 0, integrator = -1, soleJob = -1;
     int areaLights = 1;  // 0: no job of the wave has area lights (next-event rays are any-hit)
+    int interior = 0;    // 1: most paths are of interiors and keep to the scene for several bounces
     // > 0: the first bounce of units [rasterUnit0, nUnits) (paths [rasterFrom, nPaths)) may
     // be rasterised (raster_primary.cuh); raster = their per-triangle records in all
     // and rasterSamples = their samples a pixel (mean)
     int raster = 0, rasterFrom = 0, rasterUnit0 = 0, rasterSamples = 0;
 };
+// Most paths of a wave that runs in one launch by default.
+int WholeWavePaths(bool interior);
 // Launch configuration (all choices give the same films). 0 = default.
 struct WaveTuning {
     int blocksPerSm = 0;  // stage grid: blocks of 128 threads per SM (0: occupancy of the trace kernels)

@@ -185,6 +185,22 @@ int WaveAreaLights(const std::vector<DevJob>& jobs, const std::vector<WaveUnit>&
     return 0;
 }
 
+// Whether most paths of a wave are of interiors: a camera within the scene's bounds and area
+// lights. Their paths seldom leave the scene before the last bounce. Asked of waves of a fixed
+// depth of more than kShortWave iterations only: in a closed room one launch takes
+// 199,680 paths of 4 iterations in 635 us, as the stages did (629), of 5 in 828 (785; now 690).
+constexpr int kShortWave = 4;
+int WaveInterior(const std::vector<DevJob>& jobs, const std::vector<WaveUnit>& units) {
+    int64_t inside = 0, all = 0;
+    for (const WaveUnit& u : units) {
+        const DevJob& J = jobs[u.job];
+        const int64_t paths = (int64_t)J.st.width * J.st.height * u.sw;
+        if (J.inside && J.S.numLights > 0) inside += paths;
+        all += paths;
+    }
+    return 2 * inside > all ? 1 : 0;
+}
+
 int WaveSoleJob(const std::vector<WaveUnit>& units) {
     for (const WaveUnit& u : units)
         if (u.job != units.front().job) return -1;
@@ -204,6 +220,7 @@ WaveShape ShapeOf(const std::vector<DevJob>& jobs, std::vector<WaveUnit>& units,
     shape.integrator = WaveIntegrator(jobs, units);
     shape.soleJob = WaveSoleJob(units);
     shape.areaLights = WaveAreaLights(jobs, units);
+    shape.interior = shape.iters > kShortWave ? WaveInterior(jobs, units) : 0;
     PrepareRasterUnits(jobs, &units, &shape, primaryTraversal);
     return shape;
 }

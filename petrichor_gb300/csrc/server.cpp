@@ -389,6 +389,7 @@ private:
             J.S = JobScene(*r->scene, &r->job.settings);
             J.C = ToDev(&r->job.camera);
             J.st = ToDev(&r->job.settings);
+            J.inside = CameraInside(*r->scene, &r->job.camera);
             J.accum = (float4*)((char*)arena_.ptr + r->accumOff);
             J.film = r->filmHost ? (float*)((char*)arena_.ptr + r->filmOff) : r->job.film_device;
             if (e == cudaSuccess)

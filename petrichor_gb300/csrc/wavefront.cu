@@ -1070,6 +1070,12 @@ struct TailSink {
 //  - what is left of a queue-polled wave once at most kTailPaths paths are: a 256x256 16-spp
 //    Cornell frame 1755 -> 1077 us (16,384 paths 1183 us, 262,144 paths 1140 us);
 //  - the bounces from WaveTuning::tailBounce on.
+//
+// A wave of interiors (WaveShape::interior) runs whole only up to one path per thread: its paths
+// all run to the last bounce, and those beyond are a second full round. With the camera in a
+// closed room, 16 bounces, 77,000 paths among 20,000 triangles take 1.17 ms and 1.35 staged,
+// but 100,000 1.83 and 1.59, 199,680 2.93 and 2.25; among 250,000 triangles 100,000 take 2.11 and
+// 2.43, 199,680 3.32 and 3.18.
 constexpr int kTailWavePaths = 200000;
 constexpr int kTailPaths = 65536;
 constexpr int kTailBlocksPerSm = 4;  // 8 blocks: within 5% either way
@@ -1758,6 +1764,10 @@ static cudaError_t ReplayCaptured(WaveGraphCache* cache, const WaveGraphKey& key
     return cudaGraphLaunch(g->exec, stream);
 }
 
+int WholeWavePaths(bool interior) {
+    return interior ? std::min(kTailWavePaths, SmCount() * kTailBlocksPerSm * kTraceBlock) : kTailWavePaths;
+}
+
 cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& shape,
                     const WaveBuffers& wb, cudaStream_t stream, int* launches, WaveProfile* prof,
                     const WaveTuning& tune, WaveGraphCache* graphs, int lane, bool accumulate) {
@@ -1782,7 +1792,7 @@ cudaError_t RunWave(const DevJob* jobs, const WaveUnit* units, const WaveShape& 
     // the first bounce rasterised where the wave allows it (raster_primary.cuh)
     const bool sort = tune.sortRays != 0;
     const bool mayTail = !prof && !sort && tune.tailBounce >= 0;
-    const bool whole = mayTail && tune.tailBounce == 0 && shape.nPaths <= kTailWavePaths;
+    const bool whole = mayTail && tune.tailBounce == 0 && shape.nPaths <= WholeWavePaths(shape.interior != 0);
     const bool raster = !whole && shape.raster > 0 && tune.primaryTraversal != 1 && tune.sortRays == 0 &&
                         shape.iters >= 0;
     d.rasterFrom = raster ? shape.rasterFrom : shape.nPaths;

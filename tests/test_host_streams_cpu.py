@@ -14,10 +14,10 @@ def host_objects(tmp_path_factory):
     return build_host_objects(tmp_path_factory.mktemp("host"))
 
 
-def build_host_objects(out):
+def build_host_objects(out, names=("capi", "scheduler", "server", "bvh_builder")):
     """Objects of the host code behind the C ABI, to be linked with the fake runtime."""
     procs, objs = [], []
-    for name in ("capi", "scheduler", "server", "bvh_builder"):
+    for name in names:
         objs.append(str(out / f"{name}.o"))
         procs.append(subprocess.Popen(["g++", "-std=c++17", "-O1", "-ffp-contract=off", "-pthread", *includes(), "-c",
                                        os.path.join(CSRC, f"{name}.cpp"), "-o", objs[-1]]))
