@@ -391,8 +391,9 @@ typedef struct pt_tuning {
 } pt_tuning;
 /* Times candidate grids, pixel bands and graph replay on probe renders of one job
  * (its scene, camera and settings in wavefront mode, spp reduced to probe_spp; 0:
- * min(spp, 4)), then keeps the fastest for the context's later wavefront renders,
- * batches and servers. Synchronous; writes the choice to *out when not NULL. */
+ * min(spp, 4), or what makes the probe's waves run as the job's do), then keeps the
+ * fastest for the context's later wavefront renders, batches and servers. Synchronous;
+ * writes the choice to *out when not NULL. */
 int pt_autotune(pt_context* ctx, pt_scene_id scene, const pt_camera* camera,
                 const pt_settings* settings, int32_t probe_spp, pt_tuning* out);
 int pt_set_tuning(pt_context* ctx, const pt_tuning* tuning);

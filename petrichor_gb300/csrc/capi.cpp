@@ -1055,6 +1055,19 @@ int pt_autotune(pt_context* ctx, pt_scene_id scene, const pt_camera* cam, const 
     pt_settings ps = *st;
     ps.mode = PT_MODE_WAVEFRONT;
     ps.spp = probeSpp > 0 ? probeSpp : std::min(st->spp, 4);
+    if (probeSpp == 0) {
+        // enough paths to run as the render's do: a small wave takes one launch, which most of
+        // the knobs do not reach
+        const int64_t px = (int64_t)st->width * st->height;
+        std::vector<DevJob> job(1);
+        job[0].S = sg->dev;
+        job[0].st = ToDev(st);
+        job[0].inside = CameraInside(*sg, cam);
+        std::vector<WaveUnit> unit(1);
+        unit[0].sw = 1;
+        const int64_t whole = WholeWavePaths(ShapeOf(job, unit, 1).interior != 0);
+        if (px * st->spp > whole) ps.spp = (int)std::max<int64_t>(ps.spp, std::min<int64_t>(st->spp, whole / px + 1));
+    }
     ps.wave_paths = 0;
     const size_t bytes = (size_t)ps.width * ps.height * 3 * sizeof(float);
     if ((rc = Alloc(ctx, ctx->film, bytes)) != PT_OK) return rc;

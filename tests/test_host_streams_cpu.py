@@ -52,3 +52,7 @@ def test_a_render_clears_its_wave_buffers_on_its_own_stream(host_objects, tmp_pa
 def test_an_upload_needs_no_more_than_the_build_or_the_scene(host_objects, tmp_path):
     """Device memory of an upload: the larger of the build and the scene, and part of an image."""
     assert run_client(host_objects, "upload_peak.cpp", str(tmp_path / "upload_peak")).startswith("ok")
+
+
+def test_the_autotuner_probes_waves_that_run_as_the_renders(host_objects, tmp_path):
+    assert run_client(host_objects, "autotune_probe.cpp", str(tmp_path / "autotune_probe")).startswith("ok")
