@@ -93,10 +93,14 @@ struct LaneRay {
 #if PT_CHECK
     int numWide, numTris;  // bounds of nodes and tris, tested before every access
 #endif
+    template <bool kQuery>
     __device__ __forceinline__ void Start();
 };
+// kQuery: a caller's ray, which may be axis-parallel (SlabInverse).
+template <bool kQuery>
 __device__ __forceinline__ void LaneRay::Start() {
     inv = ExactRecip(d);
+    if (kQuery) inv = V3(SlabInverse(inv.x, o.x), SlabInverse(inv.y, o.y), SlabInverse(inv.z, o.z));
     tBest = tmax;
     best = -1;
     constexpr int kP = 4 * kWide;  // bytes of one plane of a node's children
@@ -363,17 +367,17 @@ __device__ __forceinline__ int LanesUsed(int n) {
 // will be loaded soon).
 // Must be called by every lane of the warp, in blocks of kTraceBlock threads.
 // kAnyHit: every ray Q loads is an any-hit ray.
-// kFixedShare, with share > 0: each warp takes `share` entries by its index instead of from
+// kQuery: the queue is a ray query's. With share > 0 each warp takes `share` entries by its index instead of from
 // the counter (QueryShare: the shares cover the queue). Two round trips to the counter fewer, and
 // its clear: 22.3 -> 16.9 us for 1000 rays at the same spread; in the wave's trace kernels the
 // extra code costs registers (an interior frame 4.28 -> 4.44 ms), so only the ray queries use it.
-template <bool kAnyHit, bool kFixedShare = false, class Q>
+template <bool kAnyHit, bool kQuery = false, class Q>
 __device__ void TraceQueue(Q& q, int n, int* fetch, int& err, int share = 0) {
     __shared__ int2 sEnt[!kAnyHit && kSmemStack > 0 ? kSmemStack * kTraceBlock : 1];
     __shared__ int sCode[kAnyHit && kSmemStack > 0 ? kSmemStack * kTraceBlock : 1];
     const int lane = threadIdx.x & 31;
     const unsigned lowerLanes = (1u << lane) - 1u;
-    const int lim = kFixedShare && share > 0 ? share : LanesUsed(n);
+    const int lim = kQuery && share > 0 ? share : LanesUsed(n);
     LaneRay r;
     int idx = -1;
     bool active = false;
@@ -391,7 +395,7 @@ __device__ void TraceQueue(Q& q, int n, int* fetch, int& err, int share = 0) {
             if (!active) idx = -1;
             const int take = min(nIdle, lim - (32 - nIdle));
             unsigned first = 0;  // past n by the warps' last fetches: more than an int for the longest queues
-            if (kFixedShare && share > 0) {
+            if (kQuery && share > 0) {
                 first = (blockIdx.x * kTraceWarps + (threadIdx.x >> 5)) * lim;
                 exhausted = true;
             } else {
@@ -406,7 +410,7 @@ __device__ void TraceQueue(Q& q, int n, int* fetch, int& err, int share = 0) {
                 const int ahead = kTraceBlock / 2 * (int)gridDim.x;
                 if (idx < n - ahead) q.Prefetch(idx + ahead);
                 q.Load(idx, r);
-                r.Start();
+                r.Start<kQuery>();
                 stk.sp = 0;
                 cur = 0;  // wide root
                 active = r.nodes != nullptr;
@@ -1012,7 +1016,7 @@ struct ShadowQueue {
 // One ray traversed by one thread (the tail kernel's form): the same node and leaf
 // order as TraceQueue gives the ray.
 __device__ __forceinline__ void TraceOne(LaneRay& r, TravStack& stk, int& err) {
-    r.Start();
+    r.Start<false>();
     stk.sp = 0;
     if (!r.nodes) return;
     int cur = 0;  // wide root
