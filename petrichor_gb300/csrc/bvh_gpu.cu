@@ -1210,6 +1210,7 @@ cudaError_t BuildBinnedSahDevice(const float* positions, int numVertices, const 
         if (hc) cudaFreeHost(hc);
         return err;
     }
+    *hc = Counters{};  // a tree of one leaf reads no counters back
     ar = Arena{static_cast<char*>(block.p), 0};
     arrays.Carve(ar, T, numVertices, nodeCap, activeCap, segCap, smallCap, heapCap);
     auto& dPos = arrays.dPos;
