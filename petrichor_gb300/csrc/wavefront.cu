@@ -355,11 +355,13 @@ __device__ __noinline__ void ResolveTie(const DevScene* S, V3 o, V3 d, float tmi
 // and 28 warps per SM; a 512x288 4-spp frame of 20,000 triangles 869 us unspread, 650, 645,
 // 650 and 666 us. (Ray queries have a spread of their own, query_share.h.)
 constexpr int kSpreadWarps = 6;
+// (In this form, for the at most 2^27 entries of a wave: with (n - 1) / warps + 1 the closest-hit
+// kernel took 71 registers instead of 64, a block less per SM and 1% of a frame.)
 __device__ __forceinline__ int LanesUsed(int n) {
     unsigned sms;
     asm("mov.u32 %0, %%nsmid;" : "=r"(sms));
     const int warps = (int)sms * kSpreadWarps;
-    return min(32, (n - 1) / warps + 1);
+    return min(32, max(1, (n + warps - 1) / warps));
 }
 
 // Q provides: void Load(int i, LaneRay&) (ray, range, and the scene: nodes = nullptr
@@ -377,7 +379,7 @@ __device__ void TraceQueue(Q& q, int n, int* fetch, int& err, int share = 0) {
     __shared__ int sCode[kAnyHit && kSmemStack > 0 ? kSmemStack * kTraceBlock : 1];
     const int lane = threadIdx.x & 31;
     const unsigned lowerLanes = (1u << lane) - 1u;
-    const int lim = kQuery && share > 0 ? share : LanesUsed(n);
+    const int lim = !kQuery ? LanesUsed(n) : share > 0 ? share : 32;
     LaneRay r;
     int idx = -1;
     bool active = false;
@@ -394,7 +396,7 @@ __device__ void TraceQueue(Q& q, int n, int* fetch, int& err, int share = 0) {
             if (!active && idx >= 0) q.Finish(idx, r);
             if (!active) idx = -1;
             const int take = min(nIdle, lim - (32 - nIdle));
-            unsigned first = 0;  // past n by the warps' last fetches: more than an int for the longest queues
+            unsigned first = 0;  // past n by the warps' last fetches: more than an int for the longest queries
             if (kQuery && share > 0) {
                 first = (blockIdx.x * kTraceWarps + (threadIdx.x >> 5)) * lim;
                 exhausted = true;
@@ -1984,7 +1986,17 @@ cudaError_t RunPrimaryHits(const DevJob* jobs, const WaveUnit* units, const Wave
     return cudaGetLastError();
 }
 
-static int TraceShare(int n) { return QueryShare(n, SmCount(), DefaultStageGrid() * kTraceWarps); }
+// Resident blocks of the query kernel (7 per SM: 4M rays take 719 us, and 733 on a grid of 8).
+static int QueryGrid() {
+    static int grid = 0;
+    if (grid == 0) {
+        int perSm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, TraceKernel, kTraceBlock, 0);
+        grid = SmCount() * std::max(1, perSm);
+    }
+    return grid;
+}
+static int TraceShare(int n) { return QueryShare(n, SmCount(), QueryGrid() * kTraceWarps); }
 bool TraceUsesCounter(int n) { return n > 0 && TraceShare(n) == 0; }
 
 cudaError_t LaunchTraceClosest(const DevScene& S, int n, const float* rays, float distMin,
@@ -1996,7 +2008,7 @@ cudaError_t LaunchTraceClosest(const DevScene& S, int n, const float* rays, floa
         const cudaError_t e = cudaMemsetAsync(fetchCounter, 0, sizeof(int), stream);
         if (e != cudaSuccess) return e;
     }
-    TraceKernel<<<DefaultStageGrid(), kTraceBlock, 0, stream>>>(S, n, rays, distMin, distMax, triOut, distOut,
+    TraceKernel<<<QueryGrid(), kTraceBlock, 0, stream>>>(S, n, rays, distMin, distMax, triOut, distOut,
                                                                 fetchCounter, share);
     return cudaGetLastError();
 }
