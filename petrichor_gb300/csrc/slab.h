@@ -41,25 +41,34 @@ PT_HD float Min3(float a, float b, float c) {
 // They are not all the boxes that such a ray meets. With a direction component of exactly zero,
 // or so small that 1 / d or o / d overflows, and an origin other than zero there, a box whose
 // planes on that axis lie on both sides of zero is left out even where it holds the origin
-// between them: one plane's distance is infinite, the other NaN. Ray queries avoid it
-// (SlabInverse). An image's paths do not: a few of the 132.7M of a 1080p frame have such a
-// direction, and may miss a hit or an occluder. Films keep their bits so.
+// between them: one plane's distance is infinite, the other NaN. Axis-parallel rays of a query
+// avoid it (SlabInverse). Other rays with one such component do not, in queries and among an image's
+// paths: about one in 3M random rays, a few of the 132.7M paths of a 1080p frame, which may miss a hit
+// or an occluder. Their results are kept bit for bit as they have been.
 PT_HD int UpperFirst(float inv, float oi) {
     const float most = 3.402823466e+38f;
     const bool over = fabsf(inv) > most || fabsf(oi) > most;
     return (copysignf(1.0f, inv) < 0.0f) != over ? 1 : 0;
 }
 
-// The reciprocal for the slab test of one axis of a caller's ray: 1 / d, or +-2^64 where it or
-// o / d overflows, a component of 2^-64 in the direction's place. A power of two times the origin is
-// exact, so a plane's distance is (plane - o) 2^64 rounded once: negative before the origin, beyond
-// any hit after it, and never NaN for coordinates below 2^64. Axis-parallel rays, the plainest of
-// picking and baking, so meet the boxes that they pass through. Once per ray; in the wave's kernels it
-// costs 1 to 2% of a frame.
-PT_HD float SlabInverse(float inv, float o) {
+// Whether 1 / d or o / d overflows.
+PT_HD bool SlabOverflows(float inv, float o) {
     const float most = 3.402823466e+38f;
-    const bool over = fabsf(inv) > most || fabsf(o * inv) > most;
-    return over ? copysignf(18446744073709551616.0f, inv) : inv;
+    return fabsf(inv) > most || fabsf(o * inv) > most;
+}
+// The reciprocal for the slab test of one axis of an axis-parallel ray: 1 / d, or +-2^64 where it
+// or o / d overflows, a component of 2^-64 in the direction's place. A power of two times the origin
+// is exact, so a plane's distance is (plane - o) 2^64 rounded once: negative before the origin,
+// beyond any hit after it, and never NaN for coordinates below 2^64. So the plainest rays of
+// picking and baking meet the boxes that they pass through. Once per ray of a query; in the wave's
+// kernels it costs 1 to 2% of a frame.
+constexpr float kSlabMost = 18446744073709551616.0f;  // 2^64
+PT_HD float SlabInverse(float inv, float o) {
+    return SlabOverflows(inv, o) ? copysignf(kSlabMost, inv) : inv;
+}
+// A ray is axis-parallel with two components below 2^-64, zero or not.
+PT_HD bool AxisParallel(float ix, float iy, float iz) {
+    return (fabsf(ix) > kSlabMost) + (fabsf(iy) > kSlabMost) + (fabsf(iz) > kSlabMost) >= 2;
 }
 
 // Entry distance of a box's overlap with [0, tmax], +infinity where there is none, from the

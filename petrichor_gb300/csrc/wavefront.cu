@@ -96,11 +96,12 @@ struct LaneRay {
     template <bool kQuery>
     __device__ __forceinline__ void Start();
 };
-// kQuery: a caller's ray, which may be axis-parallel (SlabInverse).
+// kQuery: a caller's ray, which may be axis-parallel (slab.h).
 template <bool kQuery>
 __device__ __forceinline__ void LaneRay::Start() {
     inv = ExactRecip(d);
-    if (kQuery) inv = V3(SlabInverse(inv.x, o.x), SlabInverse(inv.y, o.y), SlabInverse(inv.z, o.z));
+    if (kQuery && AxisParallel(inv.x, inv.y, inv.z))
+        inv = V3(SlabInverse(inv.x, o.x), SlabInverse(inv.y, o.y), SlabInverse(inv.z, o.z));
     tBest = tmax;
     best = -1;
     constexpr int kP = 4 * kWide;  // bytes of one plane of a node's children

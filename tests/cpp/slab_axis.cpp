@@ -57,6 +57,10 @@ int main() {
     // ordinary directions keep their reciprocal
     for (float d : {1.0f, -0.3f, 1.0e-20f, INFINITY, -INFINITY})
         if (ptg::SlabInverse(1.0f / d, 5.0f) != 1.0f / d) return std::printf("1 / %g changed\n", d), 1;
+    const float inf = INFINITY;
+    if (ptg::AxisParallel(inf, 2.0f, -1.0f) || ptg::AxisParallel(NAN, inf, 1.0f) || !ptg::AxisParallel(inf, 1.0f, -1.0e38f) ||
+        !ptg::AxisParallel(-inf, inf, 1.0f) || !ptg::AxisParallel(0.0f, -1.0e20f, inf))
+        return std::printf("axis-parallel rays mistaken\n"), 1;
     if (!std::isnan(ptg::SlabInverse(NAN, 1.0f))) return std::printf("NaN changed\n"), 1;
     std::printf("ok %ld %ld\n", cases, hits);
     return 0;
