@@ -194,7 +194,11 @@ const char* pt_last_error(const pt_context* ctx);
 int pt_camera_init(const float pos[3], const float view_dir[3], float fov, float focal_length,
                    const float* focus_target, float aperture, pt_camera* out);
 
-/* Copies the scene to the device and builds its binned-SAH BVH (kept resident). */
+/* Copies the scene to the device and builds its binned-SAH BVH (kept resident). Device memory
+ * while it runs: the build's scratch (398 bytes per triangle, 12 per vertex) beside the scene
+ * and parts of its images where there is room, else the larger of the scratch and the scene and
+ * 64 KB (host builder: the scene and 21 bytes per triangle and 36 per vertex). The budget counts the
+ * scene's own buffers. */
 int pt_scene_upload(pt_context* ctx, const pt_scene_desc* desc, pt_scene_id* out);
 int pt_scene_release(pt_context* ctx, pt_scene_id scene);
 int pt_scene_info_get(pt_context* ctx, pt_scene_id scene, pt_scene_info* info);
@@ -288,7 +292,9 @@ int pt_serve_stop(pt_context* ctx);
 
 /* Closest hits for n device rays (o.xyz, dir.xyz) within [dist_min, dist_max]:
  * original triangle index (or -1) and distance (or -1). Enqueued on `stream`; queries on
- * several streams may run at the same time (of captured ones, up to 16 of a context). */
+ * several streams may run at the same time (of captured ones, up to 16 of a context).
+ * A ray with a single direction component of exactly zero can miss a triangle whose extent
+ * on that axis holds zero; axis-parallel rays, with two, do not. */
 int pt_trace_closest(pt_context* ctx, pt_scene_id scene, int32_t n, const float* rays_device,
                      float dist_min, float dist_max, int32_t* tri_device, float* dist_device,
                      void* stream);
@@ -318,7 +324,7 @@ int pt_bvh_build(const float* positions, uint32_t num_vertices, const int32_t* i
 /* The same build on the context's GPU: the reference's tree node for node, including
  * the order std::sort leaves equal keys in. Outputs as pt_bvh_build, sized for
  * max(1, 2 * num_triangles) nodes; *num_nodes receives the count; stats may be NULL.
- * Synchronous; temporary device memory of about 250 bytes per triangle. */
+ * Synchronous; temporary device memory of 398 bytes per triangle and 12 per vertex. */
 typedef struct pt_bvh_build_stats {
   double device_ms;   /* device time, uploads to tree read back */
   int32_t levels;     /* tree levels built */

@@ -3,9 +3,11 @@
 // One wave is a set of work units (a job's sample block over all its pixels),
 // from one image or many (batched renders and the serving loop share the same
 // kernels: every path carries its job index). Each bounce runs three
-// persistent-grid kernels over compacted queues:
-//   extend : closest hit of every queued ray (binary BVH, 32 B nodes, both
-//            children's boxes fetched as one 64 B pair, ordered short stack)
+// persistent-grid kernels over compacted queues (small waves, and what is left of others, run
+// in one: TailKernel):
+//   extend : closest hit of every queued ray (4-wide BVH, a node is one 128 B line, ordered
+//            short stack in shared memory); the first bounce of pinhole cameras may be
+//            rasterised instead (raster_primary.cuh)
 //   shade  : miss / emission / surface handling of PathTracing or
 //            SimplePathTracing semantics; next-event rays go to the shadow queue,
 //            continuation rays to the next ray queue (warp-aggregated appends)
@@ -29,8 +31,8 @@ namespace ptg {
 
 // Minimum resident blocks per SM requested from the register allocator for the
 // trace (extend/shadow) stages: 7 blocks of at most 72 registers (the closest-hit kernel
-// takes 64 of them, so 8 of its blocks are resident); 8 of 64 (the others spill), 6 and 5 measured 17.65, 17.30 and 17.85 ms against 16.90 for the closest hits of the
-// 1.0M-triangle 1080p frame.
+// takes 64 of them, so 8 of its blocks are resident). The closest hits of the 1.0M-triangle
+// 1080p frame took 16.90 ms; held to 8 blocks (the other kernels spill) 17.65, to 6 17.30.
 #ifndef PT_TRACE_MIN_BLOCKS
 #define PT_TRACE_MIN_BLOCKS 7
 #endif
@@ -69,16 +71,13 @@ __device__ __forceinline__ int WarpAppend(int* counter, bool pred) {
 // costs its 150 instructions and a trip to the counter for however many lanes it fills.
 // Finished lanes keep their result until then and write all of them at once: a result's
 // reads and writes (for an area light, the whole of its contribution) stall the warp the same
-// for one lane as for twenty. With each lane's result written as its ray ended, a closed
-// interior's frame with an area light took 3.90 ms, the 1.0M-triangle 1080p frame 39.85, a
-// 2.2M-triangle 4K terrain frame 23.43 and a batch 12.65 ms; written at the refill 3.74, 39.59,
-// 23.30 and 12.54 ms, refilling at 16 lanes left. At 22, 19, 16, 14 and 12 lanes left they
-// take 3.75, 3.72, 3.73, 3.73 and 3.74; 40.79, 39.92, 39.41, 39.21 and 39.16; 23.90, 23.49, 23.23,
-// 23.11 and 23.05; 12.81, 12.63, 12.51, 12.48 and 12.47 ms; at 10 and 8 all are slower again, and
-// 4M incoherent rays with them (739 us at 12, 745 and 756).
-// Bound by issue and by the warps' own
-// latency: of 4M incoherent rays, 8 of 32 lanes were active per instruction, 70% of
-// issue slots busy and the L1 data pipe at 80%.
+// for one lane as for twenty (a room with an area light 3.90 ms a frame with each result written
+// as its ray ended, 3.74 so). Refilling with 16, 12 and 10 lanes left, the 1.0M-triangle 1080p
+// frame takes 39.41, 39.16 and more again, a 2.2M-triangle 4K terrain frame 23.23 and 23.05 ms, 4M
+// incoherent rays 739 us at 12 and 745 at 10.
+// Bound by issue and by the warps' own latency: of 4M incoherent rays 12.5 of 32 lanes are
+// active per instruction, 62% of the issue slots busy and the L1 data pipe at 90%; of a still's
+// first traced bounce 15 to 16 lanes and 66 to 74%.
 constexpr unsigned kFullMask = 0xffffffffu;
 
 struct LaneRay {
@@ -124,9 +123,8 @@ __device__ __forceinline__ void SortPair(float& ta, int& ca, float& tb, int& cb)
 // Entries of the traversal stack kept in shared memory per thread; deeper ones go
 // to local memory. Shared entries are entry-major with one column per thread of
 // the 128-thread block, so a warp's accesses always fall in 32 distinct banks. More entries
-// take from L1 and from the other stream's blocks: a 1.0M-triangle 1080p still took 40.01,
-// 39.85, 39.91 and 39.92 ms with 8, 10, 12 and 16, a 2.2M-triangle 4K terrain frame 23.54, 23.45,
-// 23.70 and 23.71 ms.
+// take from L1 and from the other stream's blocks: a 2.2M-triangle 4K terrain frame took 23.54,
+// 23.45 and 23.70 ms with 8, 10 and 12, a 1.0M-triangle 1080p still 40.01, 39.85 and 39.91 ms.
 #ifndef PT_SMEM_STACK
 #define PT_SMEM_STACK 10
 #endif
@@ -134,11 +132,9 @@ constexpr int kTraceBlock = 128;
 constexpr int kTraceWarps = kTraceBlock / 32;
 constexpr int kSmemStack = PT_SMEM_STACK;
 // A warp leaves the inner-node steps for its leaves once at most this many of its lanes
-// still hold an inner node (they wait). Stepping every lane to a leaf (0) took 18.90 ms for the
-// closest hits of the 1.0M-triangle 1080p frame where 4 took 17.77, and 787 us for 4M
-// incoherent rays where 4 took 748. With results written at the refill, 3, 4, 6 and 8 take
-// 15.47, 15.27, 15.10 and 15.15 ms (the frame 39.43, 39.18, 38.98 and 39.06), a 4K terrain
-// frame 23.20, 23.05, 22.94 and 22.98 ms, and the 4M rays 745, 740, 737 and 741 us.
+// still hold an inner node (they wait). The closest hits of the 1.0M-triangle 1080p frame take
+// 15.27, 15.10 and 15.15 ms with 4, 6 and 8, and took 6% more with 0, stepping every lane to a
+// leaf; 4M incoherent rays 740, 737 and 741 us.
 constexpr int kLeafLanes = 6;
 constexpr int kDone = INT_MIN;  // no further item (never a child code of a visited slot)
 
@@ -1987,17 +1983,9 @@ cudaError_t RunPrimaryHits(const DevJob* jobs, const WaveUnit* units, const Wave
     return cudaGetLastError();
 }
 
-// Resident blocks of the query kernel (7 per SM: 4M rays take 719 us, and 733 on a grid of 8).
-static int QueryGrid() {
-    static int grid = 0;
-    if (grid == 0) {
-        int perSm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, TraceKernel, kTraceBlock, 0);
-        grid = SmCount() * std::max(1, perSm);
-    }
-    return grid;
-}
-static int TraceShare(int n) { return QueryShare(n, SmCount(), QueryGrid() * kTraceWarps); }
+// The query kernel holds 7 blocks per SM; on the stages' grid of 8 a long query's last ones find
+// the counter at its end (4M rays 724 us on either).
+static int TraceShare(int n) { return QueryShare(n, SmCount(), DefaultStageGrid() * kTraceWarps); }
 bool TraceUsesCounter(int n) { return n > 0 && TraceShare(n) == 0; }
 
 cudaError_t LaunchTraceClosest(const DevScene& S, int n, const float* rays, float distMin,
@@ -2009,7 +1997,7 @@ cudaError_t LaunchTraceClosest(const DevScene& S, int n, const float* rays, floa
         const cudaError_t e = cudaMemsetAsync(fetchCounter, 0, sizeof(int), stream);
         if (e != cudaSuccess) return e;
     }
-    TraceKernel<<<QueryGrid(), kTraceBlock, 0, stream>>>(S, n, rays, distMin, distMax, triOut, distOut,
+    TraceKernel<<<DefaultStageGrid(), kTraceBlock, 0, stream>>>(S, n, rays, distMin, distMax, triOut, distOut,
                                                                 fetchCounter, share);
     return cudaGetLastError();
 }
