@@ -220,10 +220,12 @@ int EnsureWaveBuffers(pt_context* ctx, int capacity, cudaStream_t stream) {
     for (auto& b : ctx->wbBuffers) Free(ctx, b);
     ctx->wbBuffers.assign(1, DeviceBuffer{});
     ctx->wbCapacity = 0;
+    int* hostCount = ctx->wb.hostCount;
+    ctx->wb = WaveBuffers{};  // the status read after a render would reach the freed counters
+    ctx->wb.hostCount = hostCount;
     const size_t bytes = WaveBuffersBytesTwoLanes(capacity);
     const int rc = Alloc(ctx, ctx->wbBuffers[0], bytes);
     if (rc != PT_OK) return rc;
-    int* hostCount = ctx->wb.hostCount;
     ctx->wb = CarveWaveBuffers(ctx->wbBuffers[0].ptr, capacity);
     ctx->wb.hostCount = hostCount;
     ctx->wb.bytes = bytes;

@@ -1,4 +1,4 @@
-// A context's first wavefront render on a caller's stream, over the fake runtime: the wave
+// A context's first wavefront renders on a caller's stream, over the fake runtime: the wave
 // buffers it allocates are cleared on that stream and on no other, which nothing orders with
 // the wave's kernels. Prints "ok" or what differs.
 #include <cstdio>
@@ -65,6 +65,14 @@ int main() {
         CHECK(cleared);
     }
     CHECK(waves == 2);
+    // buffers that could not grow are gone: nothing reads the freed ones
+    st.width = st.height = 1024;
+    fake::limit = fake::inUse;
+    CHECK(pt_render_device(ctx, 1, &cam, &st, film, a) == PT_ERR_OUT_OF_MEMORY);
+    CHECK(ctx->wb.counts == nullptr || fake::blocks.count(ctx->wbBuffers[0].ptr));
+    fake::limit = 0;
+    st.width = st.height = 8;
+    CHECK(pt_render_device(ctx, 1, &cam, &st, film, a) == PT_OK && waves == 3);
     CHECK(pt_context_destroy(ctx) == PT_OK && fake::inUse == 0);
     std::printf("ok\n");
     return 0;
